@@ -144,6 +144,7 @@ struct BfsDevState {
   int32_t arm;           // explore arm chosen for the current level
   int32_t fixed_arm;     // arm used when no scheduler runs (-1 = scheduler)
   uint32_t level_cap;    // levels allowed before BFS_ERR_LEVEL_LIMIT
+  uint32_t narrow;       // 1: the loop runs narrow levels in a kernel of their own
   // learned scheduler run inside init and the last block of level
   // generation (CUDA-graph loop): it stores the next level's explore arm in
   // `arm`, which explore_any then runs

@@ -128,4 +128,34 @@ __device__ __forceinline__ int sched_pick_warp(BfsDevState *st, const LevelCount
   return arm;
 }
 
+// One warp: the learned scheduler's arm for the level with counters c, from
+// the weights w (staged in shared memory by the caller) and the graph
+// constants held in the state, stored in st->arm for explore_any.  Kept out
+// of line so that the callers' register allocation is not affected.
+static __device__ __noinline__ void fused_sched_pick(BfsDevState *st, const LevelCounters &c,
+                                               const float *w) {
+  SchedGraphConst gc;
+  gc.diam = st->sched_diam;
+  gc.avg_deg_x = st->sched_avg_deg_x;
+  sched_pick_warp<true>(st, c, w, st->sched_min_conf, gc);
+}
+
+// Copies the model to shared memory with all threads of the block: one
+// round of parallel loads instead of the MLP's dependent ones; W2 and W3 are
+// stored transposed there (sched_transposed_index), so that the warp reads
+// them without bank conflicts.  The loads
+// mark the model evict-last in L2, so that it stays there while each level's
+// edge stream (evict-first) passes through.
+// Threads first .. blockDim.x - 1 take part.
+__device__ __forceinline__ void stage_weights(float *dst, const float *__restrict__ w,
+                                              uint32_t first = 0) {
+  uint64_t pol;
+  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
+  for (uint32_t i = threadIdx.x - first; i < (uint32_t)kSchedParams; i += blockDim.x - first) {
+    float x;
+    asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(x) : "l"(w + i), "l"(pol));
+    dst[sched_transposed_index((int)i)] = x;
+  }
+}
+
 }  // namespace bfsgb

@@ -176,6 +176,7 @@ static bfs_status setup_workspace(bfs_graph *g) {
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_lg, fn, kLevelgenBlock, smem));
     g->lg_grid[par] = g->num_sms * std::max(occ_lg, 1);
   }
+  if (narrow_cluster_size(&g->narrow_cluster) != cudaSuccess) g->narrow_cluster = 0;
   // explore_any takes the hub prefix in dynamic shared memory, up to what
   // the device allows a block beside the kernel's own static arrays
   size_t static_max = 0;
@@ -376,15 +377,18 @@ static cudaError_t add_kernel(cudaGraph_t graph, cudaGraphNode_t *node,
 }
 
 // Builds the device-side level loop:
-//   fill(levels/parents, bitmaps) -> init(root) -> while(F > 0) {
-//     explore -> levelgen (last block sets the while condition) }
+//   fill(parents, working levels, bitmaps) -> init(root) -> narrow levels ->
+//   while(F > 0) { explore -> levelgen (last block sets the while condition)
+//                  -> narrow levels (sets it again) } -> level output
+// The narrow-level kernel (narrow.cu) runs consecutive levels of few edges in
+// one launch and is left out of recorded runs.
 // With a fixed arm the explore node is that arm's kernel (explore_any for the
 // GLB arms).  With arm < 0 (learned schedule) it is explore_any, which runs
 // the arm in st->arm: the scheduler runs inside init (level 0) and inside the
 // last block of level generation (the next level), so the loop has no node
 // of its own for it.  (A switch node selecting each arm's own kernel was
 // measured: about 4.5 us more per level than explore_any's uniform branch.)
-static bfs_status build_loop_graph(bfs_graph *g, int arm, int sm_factor, int ipt,
+static bfs_status build_loop_graph(bfs_graph *g, int arm, int sm_factor, int ipt, bool narrow,
                                    GraphEntry *ge) {
   cudaGraph_t graph = nullptr;
   CK(cudaGraphCreate(&graph, 0));
@@ -400,6 +404,11 @@ static bfs_status build_loop_graph(bfs_graph *g, int arm, int sm_factor, int ipt
   CK(add_kernel(graph, &n_fill, nullptr, 0, fill_kernel_fn(), g->num_sms * 4, 256, fill_args));
   void *init_args[] = {&st, &cond_arg, &one};
   CK(add_kernel(graph, &n_init, &n_fill, 1, init_kernel_fn(), 1, 32, init_args));
+  const void *narrow_fn = narrow ? narrow_kernel_fn(g->narrow_cluster, g->run_parents) : nullptr;
+  cudaGraphNode_t n_narrow = n_init;
+  if (narrow)
+    CK(add_kernel(graph, &n_narrow, &n_init, 1, narrow_fn, g->narrow_cluster, kNarrowBlock,
+                  init_args, narrow_smem_bytes(g->run_parents)));
 
   // cudaGraphNodeParams has no usable default constructor (union members)
   alignas(cudaGraphNodeParams) unsigned char wbuf[sizeof(cudaGraphNodeParams)] = {};
@@ -408,7 +417,7 @@ static bfs_status build_loop_graph(bfs_graph *g, int arm, int sm_factor, int ipt
   wp.conditional.handle = cond;
   wp.conditional.type = cudaGraphCondTypeWhile;
   wp.conditional.size = 1;
-  CK(cudaGraphAddNode(&n_while, graph, &n_init, nullptr, 1, &wp));
+  CK(cudaGraphAddNode(&n_while, graph, &n_narrow, nullptr, 1, &wp));
   cudaGraph_t body = wp.conditional.phGraph_out[0];
   cudaGraphNode_t n_out;
   CK(add_kernel(graph, &n_out, &n_while, 1, level_out_kernel_fn(), g->num_sms * 8, 256,
@@ -430,21 +439,26 @@ static bfs_status build_loop_graph(bfs_graph *g, int arm, int sm_factor, int ipt
                 g->lg_grid[g->run_parents], kLevelgenBlock, lg_args,
                 levelgen_smem(g->run_parents)));
   set_window(g, n_lg);
+  if (narrow) {
+    cudaGraphNode_t n_next;
+    CK(add_kernel(body, &n_next, &n_lg, 1, narrow_fn, g->narrow_cluster, kNarrowBlock, lg_args,
+                  narrow_smem_bytes(g->run_parents)));
+  }
   CK(cudaGraphInstantiate(&ge->exec, graph, 0));
   return BFS_OK;
 }
 
-static bfs_status get_loop_graph(bfs_graph *g, int arm, int sm_factor, int ipt,
+static bfs_status get_loop_graph(bfs_graph *g, int arm, int sm_factor, int ipt, bool narrow,
                                  GraphEntry **out) {
   const int key = (arm + 1) * 8192 + (g->run_parents ? 4096 : 0) + (ipt == 8 ? 2048 : 0) +
-                  (g->use_l2_pin ? 1024 : 0) + sm_factor;
+                  (g->use_l2_pin ? 1024 : 0) + (narrow ? 512 : 0) + sm_factor;
   auto it = g->graphs.find(key);
   if (it != g->graphs.end()) {
     *out = &it->second;
     return BFS_OK;
   }
   GraphEntry ge;
-  bfs_status rc = build_loop_graph(g, arm, sm_factor, ipt, &ge);
+  bfs_status rc = build_loop_graph(g, arm, sm_factor, ipt, narrow, &ge);
   if (rc != BFS_OK) {
     if (ge.exec) cudaGraphExecDestroy(ge.exec);
     if (ge.graph) cudaGraphDestroy(ge.graph);
@@ -616,7 +630,10 @@ bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts_
   GraphEntry *ge = nullptr;
   bfs_status rc;
   if (graph_loop) {
-    rc = get_loop_graph(g, arm, o.sm_factor, o.ipt, &ge);
+    // a recorded run takes every level through its arm's explore kernel
+    const bool narrow = g->narrow_cluster > 0 && o.record == 0;
+    s.narrow = narrow ? 1u : 0u;
+    rc = get_loop_graph(g, arm, o.sm_factor, o.ipt, narrow, &ge);
     if (rc != BFS_OK) return rc;
     if (arm < 0) {  // scheduler fused into init and level generation
       const SchedGraphConst gc = sched_graph_const(g->n_cols, g->nnz);

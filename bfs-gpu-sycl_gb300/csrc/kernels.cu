@@ -193,36 +193,6 @@ struct BlockIndex {
   static constexpr int value = B == 128 ? 0 : B == 256 ? 1 : 2;
 };
 
-// One warp: the learned scheduler's arm for the level with counters c, from
-// the weights w (staged in shared memory by the caller) and the graph
-// constants held in the state, stored in st->arm for explore_any.  Kept out
-// of line so that the callers' register allocation is not affected.
-__device__ __noinline__ void fused_sched_pick(BfsDevState *st, const LevelCounters &c,
-                                               const float *w) {
-  SchedGraphConst gc;
-  gc.diam = st->sched_diam;
-  gc.avg_deg_x = st->sched_avg_deg_x;
-  sched_pick_warp<true>(st, c, w, st->sched_min_conf, gc);
-}
-
-// Copies the model to shared memory with all threads of the block: one
-// round of parallel loads instead of the MLP's dependent ones; W2 and W3 are
-// stored transposed there (sched_transposed_index), so that the warp reads
-// them without bank conflicts.  The loads
-// mark the model evict-last in L2, so that it stays there while each level's
-// edge stream (evict-first) passes through.
-// Threads first .. blockDim.x - 1 take part.
-__device__ __forceinline__ void stage_weights(float *dst, const float *__restrict__ w,
-                                              uint32_t first = 0) {
-  uint64_t pol;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
-  for (uint32_t i = threadIdx.x - first; i < (uint32_t)kSchedParams; i += blockDim.x - first) {
-    float x;
-    asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(x) : "l"(w + i), "l"(pol));
-    dst[sched_transposed_index((int)i)] = x;
-  }
-}
-
 __device__ void init_state(BfsDevState *st, unsigned long long cond, int use_cond) {
   const uint32_t r = st->root;                     // original id
   const uint32_t ri = st->pinv ? st->pinv[r] : r;  // internal id
@@ -282,7 +252,8 @@ __global__ void init_kernel(BfsDevState *st, unsigned long long cond, int use_co
   if (w != nullptr) stage_weights(s_w, w);
   if (threadIdx.x == 0) init_state(st, cond, use_cond);
   __syncwarp();
-  if (w != nullptr) fused_sched_pick(st, level_counters(st), s_w);
+  if (w != nullptr && !narrow_next(st, st->F, st->EF))
+    fused_sched_pick(st, level_counters(st), s_w);
 }
 
 // ---- explore: LLB / SLB -----------------------------------------------------
@@ -1121,7 +1092,8 @@ __global__ void __launch_bounds__(B, kLgMinBlocks) levelgen_kernel(BfsDevState *
       s_ctr = finish_level(st, cond, use_cond);
     }
     __syncthreads();
-    if (w != nullptr && warp == 0) fused_sched_pick(st, s_ctr, s_w);
+    if (w != nullptr && warp == 0 && !narrow_next(st, s_ctr.F, s_ctr.EF))
+      fused_sched_pick(st, s_ctr, s_w);
   }
 }
 
@@ -1199,7 +1171,7 @@ __global__ void validate_vertices_kernel(uint32_t n_cols, uint32_t root,
 // every destination < n_cols.
 __global__ void check_csc_kernel(const uint32_t *__restrict__ indptr,
                                  const uint32_t *__restrict__ inds, uint32_t n_cols,
-                                 uint64_t nnz, unsigned long long *bad) {
+                                 uint64_t nnz, unsigned long long *bad, uint32_t *rows) {
   uint32_t nbad = 0;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1209,7 +1181,10 @@ __global__ void check_csc_kernel(const uint32_t *__restrict__ indptr,
   for (uint64_t k = tid; k < nnz; k += stride)
     if (inds[k] >= n_cols) nbad++;
   nbad = __reduce_add_sync(kFull, nbad);
-  if ((threadIdx.x & 31u) == 0 && nbad) atomicAdd(bad, (unsigned long long)nbad);
+  if ((threadIdx.x & 31u) == 0 && nbad) {
+    atomicAdd(bad, (unsigned long long)nbad);
+    if (rows) *rows = 0u;
+  }
 }
 
 // ---- kernel table ---------------------------------------------------------
@@ -1265,8 +1240,9 @@ cudaError_t launch_seed_state(BfsDevState *st, const BfsDevState &s, cudaStream_
 }
 
 cudaError_t launch_check_csc(const uint32_t *indptr, const uint32_t *inds, uint32_t n_cols,
-                             uint64_t nnz, unsigned long long *bad, cudaStream_t s) {
-  check_csc_kernel<<<2048, 256, 0, s>>>(indptr, inds, n_cols, nnz, bad);
+                             uint64_t nnz, unsigned long long *bad, cudaStream_t s,
+                             uint32_t *rows) {
+  check_csc_kernel<<<2048, 256, 0, s>>>(indptr, inds, n_cols, nnz, bad, rows);
   return cudaGetLastError();
 }
 

@@ -18,6 +18,39 @@ constexpr int kAnyBlock = 1024;
 constexpr int kGlbGroups = 4;
 inline uint32_t glb_chunk_edges(int ipt) { return 32u * (uint32_t)ipt * kGlbGroups; }
 
+// ---- narrow levels (narrow.cu) ----
+constexpr uint32_t kNarrowBlock = 512;
+constexpr uint32_t kNarrowHeavy = 128;       // degree of a heavy entry
+constexpr uint32_t kNarrowHeavyBound = 512;  // the same where only a bound on degrees is known
+// Largest level: 84 K edges (R-MAT scale 12) take 23 us in the two-kernel loop
+// and 14 on the cluster, 379 K (scale 14) take 86 us for the whole BFS there
+// and 101 on the cluster.
+constexpr uint32_t kNarrowEdges = 1u << 17;
+constexpr uint32_t kNarrowList = 8192;         // entries walked by the whole cluster
+constexpr uint32_t kNarrowEntries = 48u << 10;  // they fit the cluster's queues
+// Whether the narrow-level kernel takes a level of F entries and EF edges;
+// with `heavy`, `list` of them may hold many edges (or wait in global memory)
+// and are walked by the whole cluster.
+BFS_HD bool narrow_level(uint32_t F, uint32_t EF, bool heavy, uint32_t list) {
+  return F > 0u && EF <= kNarrowEdges && (heavy ? list : 0u) <= kNarrowList;
+}
+BFS_HD bool narrow_level(uint32_t F, uint32_t EF, bool heavy) {
+  return narrow_level(F, EF, heavy, F) && F <= kNarrowEntries;
+}
+// The same after init or level generation, in loops that run the kernel
+// (no entry has more than EF - F + 1 edges: each has at least one).
+BFS_HD bool narrow_next(const BfsDevState *st, uint32_t F, uint32_t EF) {
+  return st->narrow != 0u && narrow_level(F, EF, EF - F + 1u > kNarrowHeavyBound);
+}
+// Arguments (BfsDevState*, conditional_handle, use_conditional); one cluster
+// of kNarrowBlock-thread blocks, grid = cluster size,
+// narrow_smem_bytes(parents) of dynamic shared memory.
+const void *narrow_kernel_fn(int cluster, bool parents);
+size_t narrow_smem_bytes(bool parents);
+// The largest cluster (16 or 8 blocks) the current device runs the kernel
+// on; raises the kernel's attributes for it.  0 and an error if none.
+cudaError_t narrow_cluster_size(int *cluster);
+
 // Kernel function pointers (for CUDA-graph kernel nodes and direct launches).
 // Every kernel takes (BfsDevState*) first; levelgen and init also take
 // (unsigned long long conditional_handle, int use_conditional).
@@ -47,7 +80,10 @@ cudaError_t launch_validate(const uint32_t *indptr, const uint32_t *inds, uint32
                             uint32_t n_cols, uint32_t root, const int32_t *level,
                             const int32_t *parent, uint8_t *witness, uint8_t *parent_ok,
                             unsigned long long *bad, cudaStream_t s);
+// Counts the CSC's errors in *bad; where there are any and rows is given,
+// sets *rows to 0 (init then queues no root).
 cudaError_t launch_check_csc(const uint32_t *indptr, const uint32_t *inds, uint32_t n_cols,
-                             uint64_t nnz, unsigned long long *bad, cudaStream_t s);
+                             uint64_t nnz, unsigned long long *bad, cudaStream_t s,
+                             uint32_t *rows = nullptr);
 
 }  // namespace bfsgb
