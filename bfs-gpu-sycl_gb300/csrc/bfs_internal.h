@@ -90,6 +90,8 @@ BFS_HD uint32_t hash_to_range(uint64_t h, uint32_t n) {
 constexpr uint8_t kLv8Unvisited = 0xFF;
 constexpr uint8_t kLv8Deep = 0xFE;
 
+constexpr int kHubClasses = 5;  // target classes of a relabelled layout, at most
+
 struct BfsDevState {
   // graph
   const uint32_t *indptr;
@@ -125,13 +127,23 @@ struct BfsDevState {
   const uint32_t *moved; // bitmap: bit v set when perm[v] != v (null: identity)
   uint32_t hub_words;    // bitmap words of the hub prefix kept in shared memory
   uint32_t hub_min_edges;  // frontier edges from which explore loads them
+  // target classes (hub_layout.h): while every vertex of the first `skip_full`
+  // classes is visited, the entries queued leave out the edges to them, which
+  // come first in each list
+  const uint32_t *skip[kHubClasses];
+  uint32_t skip_limit[kHubClasses];
+  uint32_t skip_classes;  // 0: entries always hold all edges
+  uint32_t skip_full;     // classes found visited (written by explore)
+  uint32_t skip_min_edges;  // frontier edges from which explore looks
+  uint32_t explore_done;  // explore blocks finished this level
   // level-loop counters (written by kernels)
   unsigned long long next_packed;  // (count << 32) | chunk sum, next frontier
   unsigned long long edges_count;  // sum of degrees of expanded vertices
   uint32_t next_edges;   // degree sum of the next frontier
+  uint32_t next_walk;    // the same without the edges its entries leave out
   uint32_t cur;          // queue buffer holding the current frontier
   uint32_t F;            // current frontier entries
-  uint32_t EF;           // current frontier edges
+  uint32_t EF;           // current frontier edges (those its entries hold)
   uint32_t EC;           // current frontier 16-byte chunks of inds
   uint32_t lvl;          // level of the current frontier
   uint32_t reached;      // vertices with a level

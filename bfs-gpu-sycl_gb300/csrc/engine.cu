@@ -625,6 +625,15 @@ bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts_
     s.hub_words = g->hub->vertices / 32u;
     s.hub_min_edges = g->hub_min_edges ? g->hub_min_edges
                                        : std::max<uint32_t>(kHubMinEdges, 2u * g->hub->vertices);
+    // recorded runs report whole frontiers, and the recorder times them
+    if (o.record == 0 && timer == nullptr) {
+      s.skip_classes = g->hub->classes;
+      s.skip_min_edges = s.hub_min_edges >> 4;
+      for (uint32_t c = 0; c < g->hub->classes; c++) {
+        s.skip[c] = g->hub->skip[c];
+        s.skip_limit[c] = g->hub->limit[c];
+      }
+    }
   }
   const bool graph_loop = o.loop == BFS_LOOP_GRAPH && !timer && o.record < 2;
   GraphEntry *ge = nullptr;

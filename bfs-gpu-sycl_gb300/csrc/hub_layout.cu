@@ -20,7 +20,19 @@
 //   every other v               -> itself
 // so outside the hub prefix almost every vertex keeps its id (and the
 // locality of the original numbering).  The relabelled CSC lists, for
-// internal vertex i, the out-neighbours of perm[i] mapped through pinv.
+// internal vertex i, the out-neighbours of perm[i] mapped through pinv,
+// ordered by target class: class c holds the internal ids below limit[c] that
+// no earlier class holds, and skip[c][i] counts i's targets below limit[c].
+// Once every vertex of the first classes is visited -- on R-MAT scale 25 the
+// 2 M vertices of highest degree, which take 89 % of the edge endpoints, are
+// by the second of its two large levels -- an edge to them can reach nothing
+// new, and level generation queues a vertex without those edges, by one load
+// of skip.  About a sixteenth of the vertices are ordered by degree for this,
+// more than the shared-memory prefix holds; ordering more would cost the
+// output pass more gathers than the edges saved.  R-MAT scale 25, learned,
+// mean of 12 roots: 2.72 -> 2.07 ms (levels of 696 M and 348 M edges:
+// 1.55 -> 1.30 and 0.75 -> 0.26 ms); scale 23: 831 -> 662 us; scale 21: 379 ->
+// 279 us.
 // Level and parent arrays are still written in original ids (the level
 // generation kernel writes level[perm[v]]), so callers see no difference.
 //
@@ -127,20 +139,181 @@ __global__ void moved_kernel(const uint32_t *__restrict__ perm, uint32_t n, uint
   }
 }
 
-// One warp per internal vertex: its list is the original list of perm[i],
-// every destination mapped through pinv.
-__global__ void relabel_kernel(const uint32_t *__restrict__ indptr,
-                               const uint32_t *__restrict__ inds,
-                               const uint32_t *__restrict__ perm,
-                               const uint32_t *__restrict__ pinv,
-                               const uint32_t *__restrict__ indptr_h, uint32_t n,
-                               uint32_t *inds_h) {
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-    const uint32_t src = perm[i];
+// ---- relabelled lists ------------------------------------------------------
+// Internal vertex i's list is the list of perm[i], every destination mapped
+// through pinv and the targets ordered by class (hub_layout.h), with skip[c][i]
+// the number of targets below limit[c].
+struct Classes {
+  uint32_t n;      // classes
+  uint32_t shift;  // limit[0] = 1 << shift; every limit is 4 times the one before
+  uint32_t *skip;  // n arrays, stride apart
+  size_t stride;
+};
+
+// limit[0] = 2^s and limit[c] = 4 limit[c - 1]: the class from the top bit of
+// the id (n: no class).
+__device__ __forceinline__ uint32_t class_of(uint32_t t, const Classes &cl) {
+  const uint32_t x = t >> cl.shift;
+  const uint32_t c = x ? ((31u - __clz(x)) >> 1) + 1u : 0u;
+  return c < cl.n ? c : cl.n;
+}
+
+// Lists longer than kMidList edges take a block of 256 threads each, those
+// longer than kLongList a block of 1024.  The ids in front are ordered by
+// degree, so a warp of relabel_kernel gets 32 lists of like length: with up to
+// 4096 edges per list left to it, it took 3.5 of the build's 5.0 ms on R-MAT
+// scale 21, and 0.6 of 2.4 so.  (One warp per list whatever its length, as
+// before lists were ordered by class, took 34 of 49 ms on scale 25, where the
+// build takes 31 ms now.)
+constexpr uint32_t kMidList = 256;
+constexpr uint32_t kLongList = 8192;
+
+// One warp per 32 internal vertices: their edges in rounds of 32, whatever the
+// lists' lengths.  Two passes, counting and placing; an edge's place is its
+// rank among the warp's edges of the same vertex and class (match_any), after
+// the counts of the rounds before.
+__global__ void __launch_bounds__(256) relabel_kernel(
+    const uint32_t *__restrict__ indptr, const uint32_t *__restrict__ inds,
+    const uint32_t *__restrict__ perm, const uint32_t *__restrict__ pinv,
+    const uint32_t *__restrict__ indptr_h, uint32_t n, Classes cl, uint32_t *inds_h,
+    uint32_t *mid_list, uint32_t *long_list, uint32_t *n_list) {
+  constexpr uint32_t NW = 256 / 32, kC = kHubClasses + 1;
+  __shared__ uint32_t s_cnt[NW][32][kC];
+  __shared__ uint32_t s_in[NW][32], s_out[NW][32], s_first[NW][32];
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  const uint32_t lt = (1u << lane) - 1u, le = (2u << lane) - 1u;
+  const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  for (uint64_t i0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32u; i0 < n;
+       i0 += warps * 32u) {
+    const uint32_t i = (uint32_t)i0 + lane;
+    uint32_t b = 0, d = 0;
+    if (i < n) {
+      const uint32_t src = perm[i];
+      b = indptr[src];
+      d = indptr[src + 1] - b;
+      if (d > kMidList) {
+        const bool lng = d > kLongList;
+        (lng ? long_list : mid_list)[atomicAdd(n_list + (lng ? 1 : 0), 1u)] = i;
+        d = kNone;
+      }
+    }
+    const bool is_long = d == kNone;
+    if (is_long) d = 0;
+    const uint32_t some = __ballot_sync(kNone, d > 0u);  // vertices with edges here
+    uint32_t first = d;  // exclusive prefix of d
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+      const uint32_t y = __shfl_up_sync(kNone, first, s);
+      if (lane >= (uint32_t)s) first += y;
+    }
+    const uint32_t total = __shfl_sync(kNone, first, 31);
+    first -= d;
+    const uint32_t slot = __popc(some & lt);  // of a vertex with edges
+    const uint32_t m = __popc(some);
+    __syncwarp();
+    if (d) {
+      s_in[w][slot] = b - first;  // mod 2^32
+      s_out[w][slot] = indptr_h[i];
+      s_first[w][slot] = first;
+    }
+    if (lane < m)
+#pragma unroll
+      for (uint32_t c = 0; c < kC; c++) s_cnt[w][lane][c] = 0u;
+    __syncwarp();
+    const uint32_t start = lane < m ? s_first[w][lane] : kNone;
+    for (int pass = 0; pass < 2; pass++) {
+      uint32_t before = 0;  // vertices whose edges start before x0
+      for (uint32_t x0 = 0; x0 < total; x0 += 32u) {
+        const uint32_t x = x0 + lane, p = start - x0;
+        const uint32_t starts = __reduce_or_sync(kNone, p < 32u ? 1u << p : 0u);
+        const uint32_t o = before + __popc(starts & le) - 1u;
+        before += __popc(starts);
+        uint32_t t = 0, key = kNone;
+        if (x < total) {
+          t = pinv[inds[s_in[w][o] + x]];
+          key = o * 8u + class_of(t, cl);
+        }
+        const uint32_t same = __match_any_sync(kNone, key);
+        if (x < total) {
+          uint32_t *const cnt = &s_cnt[w][o][key & 7u];
+          const uint32_t base = pass ? *cnt : 0u;
+          if (pass) inds_h[s_out[w][o] + base + __popc(same & lt)] = t;
+        }
+        __syncwarp();
+        if (x < total && (same & lt) == 0u) s_cnt[w][o][key & 7u] += __popc(same);
+        __syncwarp();
+      }
+      if (pass == 0) {  // counts to first places
+        if (lane < m) {
+          uint32_t run = 0;
+#pragma unroll
+          for (uint32_t c = 0; c < kC; c++) {
+            const uint32_t y = s_cnt[w][lane][c];
+            s_cnt[w][lane][c] = run;
+            run += y;
+          }
+        }
+        __syncwarp();
+        if (i < n && !is_long)  // targets below limit[c]: the place of class c + 1
+          for (uint32_t c = 0; c < cl.n; c++)
+            cl.skip[c * cl.stride + i] = d ? s_cnt[w][slot][c + 1u] : 0u;
+        __syncwarp();
+      }
+    }
+  }
+}
+
+// One block per list.
+template <int B>
+__global__ void __launch_bounds__(B) relabel_long_kernel(
+    const uint32_t *__restrict__ indptr, const uint32_t *__restrict__ inds,
+    const uint32_t *__restrict__ perm, const uint32_t *__restrict__ pinv,
+    const uint32_t *__restrict__ indptr_h, uint32_t n, Classes cl, uint32_t *inds_h,
+    const uint32_t *__restrict__ long_list, const uint32_t *__restrict__ n_long) {
+  __shared__ uint32_t s_cnt[kHubClasses + 1];
+  const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+  const uint32_t total = *n_long;
+  for (uint32_t k = blockIdx.x; k < total; k += gridDim.x) {
+    const uint32_t i = long_list[k], src = perm[i];
     const uint32_t b = indptr[src], d = indptr[src + 1] - b, o = indptr_h[i];
-    for (uint32_t j = lane; j < d; j += 32u) inds_h[o + j] = pinv[inds[b + j]];
+    __syncthreads();
+    if (threadIdx.x <= cl.n) s_cnt[threadIdx.x] = 0u;
+    __syncthreads();
+    for (int pass = 0; pass < 2; pass++) {
+      uint32_t mine = 0;  // pass 0: lane c counts class c
+      for (uint32_t j0 = threadIdx.x & ~31u; j0 < d; j0 += blockDim.x) {
+        const uint32_t j = j0 + lane;
+        const uint32_t t = j < d ? pinv[inds[b + j]] : 0u;
+        const uint32_t c = j < d ? class_of(t, cl) : kNone;
+        uint32_t same = 0, num = 0;
+        for (uint32_t y = 0; y <= cl.n; y++) {
+          const uint32_t bal = __ballot_sync(kNone, c == y);
+          if (c == y) same = bal;
+          if (lane == y) num = __popc(bal);
+        }
+        if (pass == 0) {
+          mine += num;
+        } else {
+          const uint32_t base = lane <= cl.n && num ? atomicAdd(&s_cnt[lane], num) : 0u;
+          const uint32_t at = __shfl_sync(kNone, base, j < d ? c : 0u);
+          if (j < d) inds_h[o + at + __popc(same & lt)] = t;
+        }
+      }
+      if (pass == 0) {
+        if (lane <= cl.n && mine) atomicAdd(&s_cnt[lane], mine);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+          uint32_t run = 0;
+          for (uint32_t c = 0; c <= cl.n; c++) {
+            const uint32_t y = s_cnt[c];
+            s_cnt[c] = run;
+            run += y;
+            if (c < cl.n) cl.skip[c * cl.stride + i] = run;
+          }
+        }
+        __syncthreads();
+      }
+    }
   }
 }
 
@@ -150,11 +323,8 @@ void free_hub(bfs_graph *g) {
   HubLayout *h = g->hub;
   if (!h) return;
   if (h->relabelled) {
-    cudaFree(h->indptr);
+    cudaFree(h->mem);
     cudaFree(h->inds);
-    cudaFree(h->perm);
-    cudaFree(h->pinv);
-    cudaFree(h->moved);
   }
   delete h;
   g->hub = nullptr;
@@ -193,12 +363,27 @@ bfs_status build_hub(bfs_graph *g, uint32_t K) {
     g->hub = h;
     return BFS_OK;
   }
+  // Ids ordered by degree: the prefix, and for the target classes about a
+  // sixteenth of the vertices (rounded down to a power of two); the classes'
+  // limits are quarters of each other, none below 128 ids.
+  uint32_t top = 128;
+  while (top < (1u << 30) && (top * 2u <= K || top * 2u <= n / 16u)) top *= 2u;
+  const uint32_t ordered = std::min(n, std::max(K, top));
+  Classes cl = {};
+  for (uint32_t lim = top; lim >= 128u && cl.n < (uint32_t)kHubClasses && lim < n; lim >>= 2) {
+    cl.n++;
+    cl.shift = 31u - (uint32_t)__builtin_clz(lim);
+  }
+  for (uint32_t c = 0; c < cl.n; c++) h->limit[c] = 1u << (cl.shift + 2u * c);
+  h->classes = cl.n;
   h->vertices = K;
   h->relabelled = true;  // from here on the arrays below are the layout's own
   h->indptr = h->inds = nullptr;
   cudaStream_t s = g->stream;
   uint32_t *indeg = nullptr, *iota = nullptr, *sorted_deg = nullptr, *by_degree = nullptr;
   uint32_t *list_d = nullptr, *list_v = nullptr, *count = nullptr, *deg = nullptr;
+  uint32_t *mid_list = nullptr, *long_list = nullptr;
+  char *build = nullptr;
   unsigned long long *cover = nullptr, h_cover = 0;
   bool flat = false;
   uint8_t *flags = nullptr;
@@ -211,27 +396,47 @@ bfs_status build_hub(bfs_graph *g, uint32_t K) {
     e = (x);                         \
     if (e != cudaSuccess) goto done; \
   } while (0)
-  HUB_CK(dev_malloc(&h->perm, sizeof(uint32_t) * (size_t)n));
-  HUB_CK(dev_malloc(&h->pinv, sizeof(uint32_t) * (size_t)n));
-  HUB_CK(dev_malloc(&h->moved, sizeof(uint32_t) * (size_t)g->words));
-  HUB_CK(dev_malloc(&h->indptr, sizeof(uint32_t) * ((size_t)n + 1)));
-  HUB_CK(dev_malloc(&h->inds, sizeof(uint32_t) * (g->nnz ? g->nnz : 1)));
-  HUB_CK(dev_malloc(&indeg, sizeof(uint32_t) * (size_t)n));
-  HUB_CK(dev_malloc(&iota, sizeof(uint32_t) * (size_t)n));
-  HUB_CK(dev_malloc(&sorted_deg, sizeof(uint32_t) * (size_t)n));
-  HUB_CK(dev_malloc(&by_degree, sizeof(uint32_t) * (size_t)n));
-  HUB_CK(dev_malloc(&list_d, sizeof(uint32_t) * (size_t)K));
-  HUB_CK(dev_malloc(&list_v, sizeof(uint32_t) * (size_t)K));
-  HUB_CK(dev_malloc(&count, sizeof(uint32_t) * 2));
-  HUB_CK(dev_malloc(&cover, sizeof(unsigned long long)));
-  HUB_CK(dev_malloc(&deg, sizeof(uint32_t) * ((size_t)n + 1)));
-  HUB_CK(dev_malloc(&flags, 2 * (size_t)n));
-  HUB_CK(cub::DeviceRadixSort::SortPairsDescending(nullptr, t_sort, indeg, sorted_deg, iota,
-                                                   by_degree, (int64_t)n, 0, 32, s));
-  HUB_CK(cub::DeviceSelect::Flagged(nullptr, t_sel, iota, flags, list_d, count, (int64_t)n, s));
-  HUB_CK(cub::DeviceScan::ExclusiveSum(nullptr, t_scan, deg, h->indptr, (int64_t)n + 1, s));
-  tmp_bytes = std::max(t_sort, std::max(t_sel, t_scan));
-  HUB_CK(dev_malloc(&tmp, tmp_bytes));
+  // two allocations for the layout's own arrays and one for the build's (each
+  // cudaMalloc and cudaFree of its own cost the first run more than a kernel)
+  {
+    auto al = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+    const size_t v4 = al(sizeof(uint32_t) * ((size_t)n + 1)), o4 = al(sizeof(uint32_t) * (size_t)ordered);
+    const size_t mw = al(sizeof(uint32_t) * (size_t)g->words);
+    // lists of more than kMidList, kLongList edges: at most so many
+    const size_t ml = al(sizeof(uint32_t) * (size_t)(g->nnz / kMidList + 1));
+    const size_t ll = al(sizeof(uint32_t) * (size_t)(g->nnz / kLongList + 1));
+    char *p = nullptr;
+    HUB_CK(dev_malloc(&p, (3 + cl.n) * v4 + mw));
+    h->mem = p;
+    h->perm = (uint32_t *)p; p += v4;
+    h->pinv = (uint32_t *)p; p += v4;
+    h->indptr = (uint32_t *)p; p += v4;
+    h->moved = (uint32_t *)p; p += mw;
+    cl.skip = (uint32_t *)p;
+    cl.stride = v4 / sizeof(uint32_t);
+    for (uint32_t c = 0; c < cl.n; c++) h->skip[c] = cl.skip + c * cl.stride;
+    HUB_CK(dev_malloc(&h->inds, sizeof(uint32_t) * (g->nnz ? g->nnz : 1)));
+    HUB_CK(cub::DeviceRadixSort::SortPairsDescending(nullptr, t_sort, indeg, sorted_deg, iota,
+                                                     by_degree, (int64_t)n, 0, 32, s));
+    HUB_CK(cub::DeviceSelect::Flagged(nullptr, t_sel, iota, flags, list_d, count, (int64_t)n, s));
+    HUB_CK(cub::DeviceScan::ExclusiveSum(nullptr, t_scan, deg, h->indptr, (int64_t)n + 1, s));
+    tmp_bytes = std::max(t_sort, std::max(t_sel, t_scan));
+    HUB_CK(dev_malloc(&build, 5 * v4 + 2 * o4 + ml + ll + al(2 * (size_t)n) + 512 + tmp_bytes));
+    p = build;
+    indeg = (uint32_t *)p; p += v4;
+    iota = (uint32_t *)p; p += v4;
+    sorted_deg = (uint32_t *)p; p += v4;
+    by_degree = (uint32_t *)p; p += v4;
+    deg = (uint32_t *)p; p += v4;
+    list_d = (uint32_t *)p; p += o4;
+    list_v = (uint32_t *)p; p += o4;
+    mid_list = (uint32_t *)p; p += ml;
+    long_list = (uint32_t *)p; p += ll;
+    flags = (uint8_t *)p; p += al(2 * (size_t)n);
+    count = (uint32_t *)p; p += 256;
+    cover = (unsigned long long *)p; p += 256;
+    tmp = p;
+  }
 
   HUB_CK(cudaMemsetAsync(indeg, 0, sizeof(uint32_t) * (size_t)n, s));
   indeg_kernel<<<grid, 256, 0, s>>>(g->inds, g->nnz, indeg);
@@ -251,8 +456,8 @@ bfs_status build_hub(bfs_graph *g, uint32_t K) {
     flat = true;  // no hubs to speak of: no layout
     goto done;
   }
-  place_hubs_kernel<<<grid, 256, 0, s>>>(by_degree, K, h->perm, h->pinv);
-  flags_kernel<<<grid, 256, 0, s>>>(h->pinv, K, n, flags, flags + n);
+  place_hubs_kernel<<<grid, 256, 0, s>>>(by_degree, ordered, h->perm, h->pinv);
+  flags_kernel<<<grid, 256, 0, s>>>(h->pinv, ordered, n, flags, flags + n);
   HUB_CK(cudaGetLastError());
   {
     size_t t = tmp_bytes;
@@ -268,7 +473,15 @@ bfs_status build_hub(bfs_graph *g, uint32_t K) {
     size_t t = tmp_bytes;
     HUB_CK(cub::DeviceScan::ExclusiveSum(tmp, t, deg, h->indptr, (int64_t)n + 1, s));
   }
-  relabel_kernel<<<grid, 256, 0, s>>>(g->indptr, g->inds, h->perm, h->pinv, h->indptr, n, h->inds);
+  HUB_CK(cudaMemsetAsync(count + 2, 0, 2 * sizeof(uint32_t), s));
+  relabel_kernel<<<grid, 256, 0, s>>>(g->indptr, g->inds, h->perm, h->pinv, h->indptr, n, cl,
+                                      h->inds, mid_list, long_list, count + 2);
+  relabel_long_kernel<1024><<<g->num_sms, 1024, 0, s>>>(g->indptr, g->inds, h->perm, h->pinv,
+                                                        h->indptr, n, cl, h->inds, long_list,
+                                                        count + 3);
+  relabel_long_kernel<256><<<g->num_sms * 8, 256, 0, s>>>(g->indptr, g->inds, h->perm, h->pinv,
+                                                          h->indptr, n, cl, h->inds, mid_list,
+                                                          count + 2);
   HUB_CK(cudaGetLastError());
   {
     uint32_t hc[2] = {0, 0};
@@ -282,17 +495,7 @@ bfs_status build_hub(bfs_graph *g, uint32_t K) {
 done:
 #undef HUB_CK
   cudaStreamSynchronize(s);
-  cudaFree(indeg);
-  cudaFree(iota);
-  cudaFree(sorted_deg);
-  cudaFree(by_degree);
-  cudaFree(list_d);
-  cudaFree(list_v);
-  cudaFree(count);
-  cudaFree(cover);
-  cudaFree(deg);
-  cudaFree(flags);
-  cudaFree(tmp);
+  cudaFree(build);
   if (e != cudaSuccess || flat) {
     cudaGetLastError();
     g->hub = h;  // frees the layout's own arrays, never the graph's

@@ -20,6 +20,14 @@ struct HubLayout {
   uint32_t *pinv = nullptr;    // original id -> internal id
   uint32_t *moved = nullptr;   // u32[words]: bit v set when perm[v] != v
   uint32_t vertices = 0;       // K: internal ids 0 .. K-1 are the hub prefix
+  // Target classes of a relabelled layout: class c holds the internal ids
+  // below limit[c] that no class before it holds.  Every list is ordered by
+  // class (targets of no class last); skip[c][v] = targets of internal vertex
+  // v with ids below limit[c].
+  uint32_t classes = 0;
+  uint32_t limit[kHubClasses] = {};
+  uint32_t *skip[kHubClasses] = {};  // u32[n_cols] each
+  void *mem = nullptr;  // a relabelled layout's arrays but inds
   bool relabelled = false;
 };
 

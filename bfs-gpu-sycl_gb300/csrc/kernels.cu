@@ -230,6 +230,9 @@ __device__ void init_state(BfsDevState *st, unsigned long long cond, int use_con
   st->max_level = 0;
   st->next_packed = 0;
   st->next_edges = 0;
+  st->next_walk = 0;
+  st->skip_full = 0;
+  st->explore_done = 0;
   st->done_blocks = 0;
   st->lg_cursor = 0;
   st->error = 0;
@@ -603,6 +606,40 @@ __global__ void __launch_bounds__(B, 1024 / B)
                                               gridDim.x * (B / 32), nullptr, 0u);
 }
 
+// Whole grid, after a level's claims: the last block to finish looks which
+// further target classes are visited to the last vertex, for the level
+// generation that follows (it then leaves their edges out of the entries it
+// queues).  A class is a range of the visited bitmap; the search ends at the
+// first class with a vertex missing, so that it is short until it pays.
+__device__ void find_full_classes(BfsDevState *st, uint32_t full) {
+  __shared__ int s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(&st->explore_done, 1u) == gridDim.x - 1u;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  const uint4 *const vis4 = reinterpret_cast<const uint4 *>(st->vis);
+  const uint32_t classes = st->skip_classes;
+  while (full < classes) {  // limits are multiples of 128 ids
+    const uint32_t w0 = full ? st->skip_limit[full - 1u] >> 7 : 0u, w1 = st->skip_limit[full] >> 7;
+    bool all = true;
+#pragma unroll 4
+    for (uint32_t i = w0 + threadIdx.x; i < w1; i += blockDim.x) {
+      const uint4 w = __ldcg(vis4 + i);
+      all &= (w.x & w.y & w.z & w.w) == kFull;
+    }
+    if (!__syncthreads_and(all)) break;
+    full++;
+  }
+  if (threadIdx.x == 0) {
+    st->skip_full = full;
+    st->explore_done = 0u;
+  }
+}
+
 // ---- explore: any arm, chosen on the device ---------------------------------
 // One kAnyBlock-thread kernel, one block per SM, that runs any arm: the arm
 // passed in (arm_in >= 0; the GLB arms always run here, and so does every
@@ -638,7 +675,10 @@ __global__ void __launch_bounds__(kAnyBlock, 1)
     const uint32_t hw = st->hub_words;  // a multiple of 4
     // uniform over the grid; a level that reached fewer vertices than half
     // the prefix would find few hubs visited and skips the copy
-    const bool use = hw != 0 && st->EF >= st->hub_min_edges && st->reached >= hw * 16u;
+    // and so does one whose entries hold no edge to the prefix
+    const uint32_t full = st->skip_full;
+    const bool use = hw != 0 && st->EF >= st->hub_min_edges && st->reached >= hw * 16u &&
+                     (full == 0u || st->skip_limit[full - 1u] < hw * 32u);
     if (use) {
       const uint4 *src = reinterpret_cast<const uint4 *>(st->vis);
       uint4 *dst = reinterpret_cast<uint4 *>(s_hub);
@@ -648,6 +688,7 @@ __global__ void __launch_bounds__(kAnyBlock, 1)
     explore_chunk_body<kChunkGroup, PAR, true>(st, F, blockIdx.x * (kAnyBlock / 32) + (t >> 5),
                                                gridDim.x * (kAnyBlock / 32), s_hub,
                                                use ? hw * 32u : 0u);
+    if (full < st->skip_classes && st->EF >= st->skip_min_edges) find_full_classes(st, full);
   } else if (bi == 2) {
     const uint32_t v = t >> 9, o = v * 513u;
     if (form == BFS_LB_SLB)
@@ -688,12 +729,13 @@ __device__ LevelCounters finish_level(BfsDevState *st, unsigned long long cond, 
   const unsigned long long packed = *(volatile unsigned long long *)&st->next_packed;
   const uint32_t f_new = (uint32_t)(packed >> 32);
   const uint32_t ec_new = (uint32_t)packed;
-  const uint32_t ef_new = *(volatile uint32_t *)&st->next_edges;
+  const uint32_t ef_new = *(volatile uint32_t *)&st->next_walk;
+  const uint32_t edges_new = *(volatile uint32_t *)&st->next_edges;
   const uint32_t lvl = st->lvl + 1;
   const uint32_t reached = *(volatile uint32_t *)&st->reached;
   if (reached > st->reached_prev) st->max_level = lvl;
   st->reached_prev = reached;
-  st->edges_count += ef_new;
+  st->edges_count += edges_new;
   const uint32_t nq = st->cur ^ 1u;
   st->qc[nq][f_new] = ec_new;  // trailing total of the new queue's scan
   st->cur = nq;
@@ -703,6 +745,7 @@ __device__ LevelCounters finish_level(BfsDevState *st, unsigned long long cond, 
   st->lvl = lvl;
   st->next_packed = 0;
   st->next_edges = 0;
+  st->next_walk = 0;
   st->done_blocks = 0;
   st->lg_cursor = 0;
   st->launches += 2;
@@ -780,6 +823,7 @@ __global__ void __launch_bounds__(B, kLgMinBlocks) levelgen_kernel(BfsDevState *
   __shared__ uint32_t s_wc[2][NW];
   __shared__ unsigned long long s_wtot[NW];
   __shared__ uint32_t s_wdeg[NW];
+  __shared__ uint32_t s_wwalk[NW];
   __shared__ uint32_t s_wreach[NW];
   __shared__ unsigned long long s_base;
   __shared__ uint32_t s_sb[2];
@@ -811,7 +855,10 @@ __global__ void __launch_bounds__(B, kLgMinBlocks) levelgen_kernel(BfsDevState *
                        0x01010101u;  // the new level in every byte
   // new vertices and kept entries' degrees counted by this lane (summed over
   // the block at the end)
-  uint32_t my_reached = 0, my_deg = 0;
+  uint32_t my_reached = 0, my_deg = 0, my_walk = 0;
+  // edges to the first skip_full classes are left out of the entries
+  const uint32_t full = st->skip_full;
+  const uint32_t *__restrict__ skip = full ? st->skip[full - 1u] : nullptr;
 
   // the working levels of word w with new bits x: sector (l0, l1) merged and
   // written back; a deep level also goes to the output (original ids)
@@ -839,10 +886,10 @@ __global__ void __launch_bounds__(B, kLgMinBlocks) levelgen_kernel(BfsDevState *
   // issued before their first use; kept entries (degree > 0) are compacted
   // in place, in list order, to [lo, lo + count) -- positions only move down
   // and an iteration's entries are already in registers.  Returns the warp's
-  // kept count, degree and chunk sums (uniform over the warp).
-  auto pass1 = [&](uint32_t lo, uint32_t hi, uint32_t &n_cnt, uint32_t &n_deg,
-                   uint32_t &n_chk) {
-    n_cnt = n_deg = n_chk = 0;
+  // kept count and chunk sum (uniform over the warp).
+  auto pass1 = [&](uint32_t lo, uint32_t hi, uint32_t &n_cnt, uint32_t &n_chk) {
+    n_cnt = n_chk = 0;
+    uint32_t n_left = 0;
     for (uint32_t t0 = lo; t0 < hi; t0 += 32u * kLgUnroll) {
       uint32_t b[kLgUnroll], e[kLgUnroll], o[kLgUnroll];
 #pragma unroll
@@ -857,6 +904,11 @@ __global__ void __launch_bounds__(B, kLgMinBlocks) levelgen_kernel(BfsDevState *
           if (v < n_rows) {
             b[r] = indptr[v];
             e[r] = indptr[v + 1];
+            if (skip) {
+              const uint32_t x = skip[v];
+              b[r] += x;
+              n_left += x;
+            }
           }
         }
       }
@@ -871,11 +923,12 @@ __global__ void __launch_bounds__(B, kLgMinBlocks) levelgen_kernel(BfsDevState *
           if (PAR) s_o[p] = o[r];
         }
         n_cnt += __popc(km);
-        n_deg += deg;
+        my_walk += deg;
+        my_deg += deg;
         n_chk += edge_chunks(b[r], deg, off);
       }
     }
-    n_deg = __reduce_add_sync(kFull, n_deg);
+    my_deg += n_left;
     n_chk = __reduce_add_sync(kFull, n_chk);
   };
   // Pass 2 (one warp): the n_cnt kept entries at [lo, lo + n_cnt) to queue
@@ -969,12 +1022,9 @@ __global__ void __launch_bounds__(B, kLgMinBlocks) levelgen_kernel(BfsDevState *
       __syncthreads();
       // this warp's share of the list
       const uint32_t lo = (L * warp) / NW, hi = (L * (warp + 1u)) / NW;
-      uint32_t n_cnt, n_deg, n_chk;
-      pass1(lo, hi, n_cnt, n_deg, n_chk);
-      if (lane == 0) {
-        s_wtot[warp] = ((unsigned long long)n_cnt << 32) | n_chk;
-        s_wdeg[warp] = n_deg;
-      }
+      uint32_t n_cnt, n_chk;
+      pass1(lo, hi, n_cnt, n_chk);
+      if (lane == 0) s_wtot[warp] = ((unsigned long long)n_cnt << 32) | n_chk;
       __syncthreads();
       if (threadIdx.x == 0) {
         unsigned long long run = 0;
@@ -982,7 +1032,6 @@ __global__ void __launch_bounds__(B, kLgMinBlocks) levelgen_kernel(BfsDevState *
           const unsigned long long y = s_wtot[i];
           s_wtot[i] = run;
           run += y;
-          my_deg += s_wdeg[i];
         }
         s_base = run ? atomicAdd(&st->next_packed, run) : 0ull;
       }
@@ -997,14 +1046,11 @@ __global__ void __launch_bounds__(B, kLgMinBlocks) levelgen_kernel(BfsDevState *
     const uint32_t lo = warp * kSlice;  // this warp's slice of the list
     uint32_t size = 0;                  // entries in the slice
     auto flush = [&]() {
-      uint32_t n_cnt, n_deg, n_chk;
-      pass1(lo, lo + size, n_cnt, n_deg, n_chk);
+      uint32_t n_cnt, n_chk;
+      pass1(lo, lo + size, n_cnt, n_chk);
       if (n_cnt) {
         unsigned long long wb = 0;
-        if (lane == 0) {
-          wb = atomicAdd(&st->next_packed, ((unsigned long long)n_cnt << 32) | n_chk);
-          my_deg += n_deg;
-        }
+        if (lane == 0) wb = atomicAdd(&st->next_packed, ((unsigned long long)n_cnt << 32) | n_chk);
         pass2(lo, n_cnt, __shfl_sync(kFull, wb, 0));
       }
       size = 0;
@@ -1061,20 +1107,25 @@ __global__ void __launch_bounds__(B, kLgMinBlocks) levelgen_kernel(BfsDevState *
   // the time it knows it is last.  Thread 0 stays out of the copy: its fence
   // would otherwise wait for its share of the loads.
   my_reached = __reduce_add_sync(kFull, my_reached);
+  my_deg = __reduce_add_sync(kFull, my_deg);
+  my_walk = __reduce_add_sync(kFull, my_walk);
   if (lane == 0) {
     s_wreach[warp] = my_reached;
     s_wdeg[warp] = my_deg;
+    s_wwalk[warp] = my_walk;
   }
   __syncthreads();  // also: every warp is done with the list
   const float *w = st->sched_w;
   float *s_w = reinterpret_cast<float *>(s_dyn);
   if (threadIdx.x == 0) {
-    uint32_t reached = 0, deg_sum = 0;
+    uint32_t reached = 0, deg_sum = 0, walk = 0;
 #pragma unroll
     for (int i = 0; i < NW; i++) {
       reached += s_wreach[i];
       deg_sum += s_wdeg[i];
+      walk += s_wwalk[i];
     }
+    if (walk) atomicAdd(&st->next_walk, walk);
     if (deg_sum) atomicAdd(&st->next_edges, deg_sum);  // a total: order does not matter
     if (reached) atomicAdd(&st->reached, reached);
     __threadfence();

@@ -75,8 +75,10 @@ typedef struct bfs_options {
   int32_t sm_factor;   /* blocks per SM for the persistent grid (0 = auto) */
   int32_t loop;        /* bfs_loop */
   int32_t l2_pin;      /* 1 = pin the visited bitmaps in L2 (default on) */
-  int32_t record;      /* 1 = fill bfs_stats per-level arrays; 2 = also time
-                          every kernel with CUDA events (forces the host loop) */
+  int32_t record;      /* 1 = fill bfs_stats per-level arrays (every level then
+                          runs its arm's explore kernel on its whole frontier);
+                          2 = also time every kernel with CUDA events (forces
+                          the host loop) */
   int32_t ipt;         /* edges per lane in flight in the explore kernels:
                           4 or 8 (0 = 4) */
 } bfs_options;
@@ -142,8 +144,12 @@ bfs_status bfs_graph_device_csc(const bfs_graph *g, const uint32_t **d_indptr,
  * original numbering, since their tile-local balancing suffers when the hubs
  * are consecutive ids.  Levels, parents and every other entry point still
  * use the caller's ids; results are identical with or without the layout.  The copy
- * costs nnz + 3 n_cols + 1 uint32 of device memory; if it cannot be
- * allocated the handle runs without it.
+ * costs nnz + 8 n_cols + 1 uint32 of device memory; if it cannot be
+ * allocated the handle runs without it.  The copy's lists are ordered by the
+ * targets' degree class; once all vertices of the highest classes are
+ * visited, the frontier leaves out the edges to them, which can reach nothing
+ * new (recorded runs keep whole frontiers).  edges_count is the same either
+ * way.
  * vertices: -1 = automatic (the default: K = 2^18, capped by the device's
  * shared memory), 0 = off, > 0 = K (rounded down to a multiple of 128).
  * min_edges: the smallest level (frontier edges) for which the explore
