@@ -47,19 +47,19 @@
 
 namespace bfsgb {
 
-// Claim of bit n after a plain load saw it clear (the load may see a stale 0
-// from an L1 copy; atomicOr's return value is authoritative, so exactly one
-// thread claims n).  Parents are written in original ids (perm: internal ->
-// original, null for the identity); `from` already is one.
+// Claim of bit n after a load in this kernel saw it clear: a reduction, no
+// value comes back.  The load may be a stale L1 copy of a word that another
+// edge of this level has claimed n in since, never of one from before this
+// kernel: whoever claims, n was not visited before this level and `from` is in
+// its frontier, so each claimer's parent is a right one and the last store
+// stays.  (A returning atomicOr that lets one claimer through costs the
+// same on R-MAT scale 25 as long as claims are made slot by slot: 8.1 and
+// 8.4 ms.)  Parents are written in original ids (perm:
+// internal -> original, null for the identity); `from` already is one.
 __device__ __forceinline__ void claim(uint32_t *vis, uint32_t n, int32_t *parent, uint32_t from,
                                       const uint32_t *perm) {
-  const uint32_t w = n >> 5, bit = 1u << (n & 31u);
-  if (parent) {
-    const uint32_t old = atomicOr(vis + w, bit);
-    if (!(old & bit)) parent[perm ? perm[n] : n] = (int32_t)from;
-  } else {
-    red_or(vis + w, bit);  // result unused: a reduction, no round trip
-  }
+  red_or(vis + (n >> 5), 1u << (n & 31u));
+  if (parent) parent[perm ? perm[n] : n] = (int32_t)from;
 }
 
 // Test-then-claim of bit n.
@@ -416,15 +416,19 @@ __global__ void __launch_bounds__(B, (MinBlocks<B, U, STRIDED>::value))
 // then set in s_hub for the block's later probes (bits only ever go from 0
 // to 1, so any snapshot is a valid "already visited" set).
 // Chunks per lane and group of the chunk walk, whatever the ipt option: with
-// the next group's loads in flight that is 16 edge slots per lane, at the
-// 64 registers of a 1024-thread block (4 chunks per group spill).
-constexpr int kChunkGroup = 2;
+// the next group's loads in flight, two chunks are 16 edge slots per lane, at
+// the 64 registers of a 1024-thread block (4 chunks per group spill).  One
+// chunk does better where a warp has few groups to walk or entries of few
+// chunks: R-MAT scale 19 173 us (GLB) instead of 199 with two, scale 21 253
+// instead of 272, ER 3 M vertices 413 instead of 430; scale 23 615 either way;
+// scale 25 2.00 ms instead of 1.92.  So levels from kGroupChunks on walk two.
+constexpr uint32_t kGroupChunks = 1u << 25;
 
 template <int U, bool PAR, bool HUB>
 __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict__ st,
                                                    uint32_t F, uint32_t gw,
                                                    uint32_t total_warps, uint32_t *s_hub,
-                                                   uint32_t hub_lim) {
+                                                   uint32_t hub_lim, uint2 *s_claim) {
   constexpr uint32_t kRound = 32u * U;
   constexpr uint32_t kMinChunk = kRound * kGlbGroups;
   const uint32_t EC = st->EC;
@@ -448,8 +452,24 @@ __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t le_mask = (2u << lane) - 1u;  // lanes 0 .. lane (all for lane 31)
   const uint64_t pol = evict_first_policy();
-  // about four warp chunks per warp, whole groups of U rounds
-  uint64_t ch = ((uint64_t)EC + 4ull * total_warps - 1) / (4ull * total_warps);
+  // Claims wait in the warp's 32 slots of s_claim (target, queue entry) and
+  // are made 32 at a time, with the parents' chain of loads and the store
+  // side by side.  Made slot by slot, with a few lanes each, they took R-MAT
+  // scale 25 with parents from 4.0 to 8.4 ms per BFS (scale 23 0.91 to 1.70,
+  // scale 21 0.33 to 0.50), and without parents from 1.96 to 2.09.
+  uint32_t waiting = 0;
+  auto flush_claims = [&]() {
+    __syncwarp();
+    if (lane < waiting) {
+      const uint2 c = s_claim[lane];
+      claim(vis, c.x, parent, PAR ? qv[c.y] : 0u, perm);
+      if (HUB && c.x < hub_lim) atomicOr(s_hub + (c.x >> 5), 1u << (c.x & 31u));
+    }
+    __syncwarp();
+    waiting = 0;
+  };
+  // about eight warp chunks per warp, whole groups of U rounds
+  uint64_t ch = ((uint64_t)EC + 8ull * total_warps - 1) / (8ull * total_warps);
   ch = (ch + kRound - 1) / kRound * kRound;
   const uint32_t CHUNK = (uint32_t)(ch > kMinChunk ? ch : kMinChunk);
   const uint32_t n_chunks = (uint32_t)(((uint64_t)EC + CHUNK - 1) / CHUNK);
@@ -463,19 +483,17 @@ __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict
     uint32_t cb = qb[cur] + off;
     uint32_t ce = cb + qd[cur];
     uint32_t cd = (cb >> 2) - qc[cur];
-    uint32_t cv = PAR ? qv[cur] : 0u;
     // window: entries c0 + 1 .. c0 + 32, one per lane (chunk start, offset,
-    // edge range, id); re-based only when a round could leave it
-    uint32_t c0 = cur, bnd, wd, wb, we, wv;
+    // edge range); re-based only when a round could leave it
+    uint32_t c0 = cur, bnd, wd, wb, we;
     auto load_window = [&]() {
       const uint32_t j = c0 + 1u + lane;
       bnd = (j <= F) ? qc[j] : kFull;  // qc[F] = EC
-      wb = we = wd = wv = 0u;
+      wb = we = wd = 0u;
       if (j < F) {
         wb = qb[j] + off;
         we = wb + qd[j];
         wd = (wb >> 2) - bnd;
-        if (PAR) wv = qv[j];
       }
     };
     load_window();
@@ -500,9 +518,8 @@ __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict
         const uint32_t sd = __shfl_sync(kFull, wd, srcl);
         const uint32_t sb = __shfl_sync(kFull, wb, srcl);
         const uint32_t se = __shfl_sync(kFull, we, srcl);
-        const uint32_t sv = PAR ? __shfl_sync(kFull, wv, srcl) : 0u;
         const uint32_t d = k ? sd : cd, b = k ? sb : cb, e = k ? se : ce;
-        fr[u] = PAR ? (k ? sv : cv) : 0u;
+        fr[u] = PAR ? cur + k : 0u;
         m[u] = 0u;
         q[u] = make_uint4(0u, 0u, 0u, 0u);
         if (x < w1) {
@@ -529,7 +546,6 @@ __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict
           cd = __shfl_sync(kFull, wd, sl);
           cb = __shfl_sync(kFull, wb, sl);
           ce = __shfl_sync(kFull, we, sl);
-          if (PAR) cv = __shfl_sync(kFull, wv, sl);
         }
       }
     };
@@ -537,9 +553,8 @@ __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict
     // predicated shared load of the hub word (hub ids only), then a
     // predicated global load of the visited word (valid slots the hub word
     // did not show visited); a slot whose word shows its bit clear gets a
-    // bit in need[u].  Only then, behind one branch per chunk, the claims --
-    // a claim is an asm statement that orders memory, so no load may follow
-    // it within the group.
+    // bit in need[u].  Only then, behind one branch per chunk, the claims,
+    // packed into the warp's waiting slots.
     auto probe = [&](const uint4 (&q)[U], const uint32_t (&m)[U], const uint32_t (&fr)[U]) {
       uint32_t need[U];
 #pragma unroll
@@ -563,14 +578,16 @@ __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict
       }
 #pragma unroll
       for (int u = 0; u < U; u++) {
-        if (need[u] == 0u) continue;
+        if (!__any_sync(kFull, need[u] != 0u)) continue;
         const uint32_t n4[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-          if (!((need[u] >> i) & 1u)) continue;
-          const uint32_t n = n4[i];
-          claim(vis, n, parent, fr[u], perm);
-          if (HUB && n < hub_lim) atomicOr(s_hub + (n >> 5), 1u << (n & 31u));
+          const uint32_t bal = __ballot_sync(kFull, (need[u] >> i) & 1u);
+          const uint32_t num = __popc(bal);
+          if (waiting + num > 32u) flush_claims();  // uniform
+          if ((need[u] >> i) & 1u)
+            s_claim[waiting + __popc(bal & (le_mask >> 1))] = make_uint2(n4[i], fr[u]);
+          waiting += num;
         }
       }
     };
@@ -592,6 +609,7 @@ __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict
       }
     }
   }
+  flush_claims();
 }
 
 // The GLB arms' own kernel (the engine runs GLB levels in explore_any; the
@@ -602,8 +620,10 @@ __global__ void __launch_bounds__(B, 1024 / B)
   const uint32_t F = st->F;
   if (F == 0) return;
   note_arm<1 * 3 + BlockIndex<B>::value>(st);
-  explore_chunk_body<kChunkGroup, PAR, false>(st, F, blockIdx.x * (B / 32) + (threadIdx.x >> 5),
-                                              gridDim.x * (B / 32), nullptr, 0u);
+  __shared__ uint2 s_claim[B];
+  explore_chunk_body<1, PAR, false>(st, F, blockIdx.x * (B / 32) + (threadIdx.x >> 5),
+                                    gridDim.x * (B / 32), nullptr, 0u,
+                                    s_claim + (threadIdx.x & ~31u));
 }
 
 // Whole grid, after a level's claims: the last block to finish looks which
@@ -659,8 +679,9 @@ __global__ void __launch_bounds__(kAnyBlock, 1)
     explore_any_kernel(BfsDevState *__restrict__ st, int arm_in) {
   extern __shared__ __align__(16) uint32_t s_hub[];
   __shared__ uint32_t s_off[kAnyBlock + 8];
-  __shared__ uint32_t s_dif[kAnyBlock];
-  __shared__ uint32_t s_vid[kAnyBlock];
+  __shared__ __align__(8) uint32_t s_two[2 * kAnyBlock];
+  uint32_t *const s_dif = s_two, *const s_vid = s_two + kAnyBlock;  // LLB, SLB
+  uint2 *const s_claim = reinterpret_cast<uint2 *>(s_two);          // GLB: the warps' claims
   __shared__ uint32_t s_wsum[kAnyBlock / 32];
   const uint32_t F = st->F;
   if (F == 0) return;
@@ -685,9 +706,12 @@ __global__ void __launch_bounds__(kAnyBlock, 1)
       for (uint32_t i = t; i < (hw >> 2); i += kAnyBlock) dst[i] = src[i];
       __syncthreads();
     }
-    explore_chunk_body<kChunkGroup, PAR, true>(st, F, blockIdx.x * (kAnyBlock / 32) + (t >> 5),
-                                               gridDim.x * (kAnyBlock / 32), s_hub,
-                                               use ? hw * 32u : 0u);
+    const uint32_t gw = blockIdx.x * (kAnyBlock / 32) + (t >> 5);
+    const uint32_t gws = gridDim.x * (kAnyBlock / 32), lim = use ? hw * 32u : 0u;
+    if (st->EC >= kGroupChunks)
+      explore_chunk_body<2, PAR, true>(st, F, gw, gws, s_hub, lim, s_claim + (t & ~31u));
+    else
+      explore_chunk_body<1, PAR, true>(st, F, gw, gws, s_hub, lim, s_claim + (t & ~31u));
     if (full < st->skip_classes && st->EF >= st->skip_min_edges) find_full_classes(st, full);
   } else if (bi == 2) {
     const uint32_t v = t >> 9, o = v * 513u;
