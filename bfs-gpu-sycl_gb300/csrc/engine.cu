@@ -326,6 +326,8 @@ static int host_blocks(const bfs_graph *g, int arm, int sm_factor, int ipt, uint
     want = (chunks + (B / 32) - 1) / (B / 32);
   } else {
     want = ((uint64_t)F + B - 1) / B;
+    // LLB's ranges are edges, not entries
+    if (arm_lb(arm) == BFS_LB_LLB) want = std::max<uint64_t>(want, EF / (4u * B) + 1);
   }
   return (int)std::max<uint64_t>(
       1, std::min<uint64_t>(want, persistent_blocks(g, arm, sm_factor, ipt)));
