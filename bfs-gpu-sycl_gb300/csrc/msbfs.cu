@@ -26,10 +26,11 @@
 //             scattered partial-sector stores, which HBM turns into
 //             read-modify-writes); kept vertices are compacted with
 //             ballot/popc and one atomic per block.
-//   expand    one warp per 32 vertices writes every root's 32 level entries
-//             as one 128-byte segment (-1 where unreached), once per pass; if
+//   expand    one warp per 128 vertices and 32 roots writes each root's 128
+//             level entries as one run (-1 where unreached), once per pass; if
 //             the search goes past the history it runs at that point and the
-//             deeper levels are stored into the rows directly.
+//             deeper levels are stored into the rows directly.  Its launch in
+//             the loop also looks which target classes every root has reached.
 //   loop      a CUDA graph with a conditional WHILE node, as for one root.
 //
 // With the graph handle's hub layout (hub_layout.cu) the batch runs on the
@@ -39,8 +40,11 @@
 // copies it into shared memory on large levels and skips the 8-byte mask
 // probe of those targets -- on power-law graphs many edges of the later
 // levels point at them, and the mask array is larger than L2, so each probe
-// skipped is a DRAM sector saved.  Rows are written in original ids (expand reads the internal state
-// through pinv).
+// skipped is a DRAM sector saved.  Once every root has reached all vertices
+// of the highest target classes, entries are queued without their edges to
+// them, as in the single-root path (R-MAT scale 22, the third of the three
+// large explore levels 400 -> 264 us; scale 25, 3.7 -> 2.2 ms).  Rows are
+// written in original ids (expand reads the internal state through pinv).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -86,6 +90,13 @@ struct MsState {
   uint32_t *hubfull;       // bit v (v < 32 hub_words): every root has reached v
   uint32_t hub_words;      // words of hubfull (0: no filter)
   uint32_t hub_min_edges;  // frontier edges from which explore loads it
+  // target classes (hub_layout.h): entries leave out the edges to classes
+  // that every root of the pass has reached to the last vertex
+  const uint32_t *skip[kHubClasses];
+  uint32_t skip_limit[kHubClasses];
+  uint32_t skip_classes;
+  uint32_t full;      // classes known to be reached by every root
+  uint32_t not_full;  // bit c: class c has a vertex some root has not reached
   uint32_t n_lanes;
   uint32_t roots[kLanes];
   unsigned long long next_packed;
@@ -95,38 +106,54 @@ struct MsState {
   unsigned long long edges[kLanes];
 };
 
-// One block of 64 threads: seeds every root and builds the first frontier
-// (roots shared by several lanes become one entry with several mask bits).
-__global__ void ms_init_kernel(MsState *st, unsigned long long cond, int use_cond) {
-  const uint32_t j = threadIdx.x;
+// One block of 64 threads, one per root: seeds the root; the first thread of
+// each distinct root with edges makes its entry, with the bits of all threads
+// that share it.  (One thread going through the roots in turn took 125 us.)
+__global__ void __launch_bounds__(kLanes) ms_init_kernel(MsState *st, unsigned long long cond,
+                                                         int use_cond) {
+  __shared__ uint32_t s_root[kLanes], s_deg[kLanes];
+  const uint32_t j = threadIdx.x, nl = st->n_lanes;
   const uint32_t *pinv = st->pinv;  // roots are original ids
-  if (j < st->n_lanes) {
-    const uint32_t r = pinv ? pinv[st->roots[j]] : st->roots[j];
+  uint32_t r = kFull, b = 0, deg = 0;
+  if (j < nl) {
+    r = pinv ? pinv[st->roots[j]] : st->roots[j];
     atomicOr(&st->vis[r], 1ull << j);
     atomicOr(&st->prev[r], 1ull << j);
     atomicOr(&st->hist[r], 1ull << j);  // level 0
-  }
-  if (j < kLanes) st->edges[j] = 0;
-  __syncthreads();
-  if (j == 0) {
-    uint32_t F = 0, EF = 0;
-    for (uint32_t l = 0; l < st->n_lanes; l++) {
-      const uint32_t r = pinv ? pinv[st->roots[l]] : st->roots[l];
-      if (r >= st->n_rows) continue;
-      const uint32_t b = st->indptr[r], e = st->indptr[r + 1];
-      if (e == b) continue;
-      uint32_t k = 0;
-      while (k < F && st->qb[0][k] != b) k++;  // same root -> same first edge
-      if (k < F) {
-        st->qm[0][k] |= 1ull << l;
-        continue;
-      }
-      st->qb[0][F] = b;
-      st->qp[0][F] = EF;
-      st->qm[0][F] = 1ull << l;
-      EF += e - b;
-      F++;
+    if (r < st->n_rows) {
+      b = st->indptr[r];
+      deg = st->indptr[r + 1] - b;
     }
+  }
+  s_root[j] = r;
+  __syncthreads();
+  unsigned long long mask = 0;
+  bool first = true;
+  for (uint32_t l = 0; l < nl; l++) {
+    const bool same = s_root[l] == r;
+    mask |= same ? 1ull << l : 0ull;
+    first &= !(same && l < j);
+  }
+  if (!first) deg = 0;
+  s_deg[j] = deg;
+  __syncthreads();
+  uint32_t slot = 0, before = 0, F = 0, EF = 0;
+  for (uint32_t l = 0; l < nl; l++) {
+    const uint32_t d = s_deg[l];
+    if (l < j) {
+      slot += d ? 1u : 0u;
+      before += d;
+    }
+    F += d ? 1u : 0u;
+    EF += d;
+  }
+  if (deg) {
+    st->qb[0][slot] = b;
+    st->qp[0][slot] = before;
+    st->qm[0][slot] = mask;
+  }
+  st->edges[j] = 0;
+  if (j == 0) {
     st->qp[0][F] = EF;
     st->F = F;
     st->EF = EF;
@@ -137,6 +164,8 @@ __global__ void ms_init_kernel(MsState *st, unsigned long long cond, int use_con
     st->error = 0;
     st->max_level = 0;
     st->any_new = 0;
+    st->full = 0;
+    st->not_full = 0;
     st->launches = 2;  // memset, init
     if (use_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond, F > 0);
   }
@@ -158,7 +187,9 @@ __global__ void __launch_bounds__(kMsBlock, 1536 / kMsBlock)
   if (F == 0) return;
   const uint32_t EF = st->EF;
   const uint32_t hw = st->hub_words;  // a multiple of 4
-  const bool use_hub = hw != 0 && EF >= st->hub_min_edges;  // uniform over the grid
+  // uniform over the grid; no entry holds an edge to a class left out
+  const bool use_hub = hw != 0 && EF >= st->hub_min_edges &&
+                       (st->full == 0u || st->skip_limit[st->full - 1u] < hw * 32u);
   if (use_hub) {
     const uint4 *src = reinterpret_cast<const uint4 *>(st->hubfull);
     uint4 *dst = reinterpret_cast<uint4 *>(s_full);
@@ -237,6 +268,13 @@ __global__ void __launch_bounds__(kMsBlock, 1536 / kMsBlock)
   }
 }
 
+// Classes reached by every root, after ms_between_classes has looked.
+__device__ __forceinline__ uint32_t ms_full_classes(const MsState *st) {
+  const uint32_t nf = st->not_full;
+  const uint32_t first = nf ? (uint32_t)__ffs(nf) - 1u : st->skip_classes;
+  return first < st->skip_classes ? first : st->skip_classes;
+}
+
 __device__ void ms_finish(MsState *st, unsigned long long cond, int use_cond) {
   const unsigned long long packed = *(volatile unsigned long long *)&st->next_packed;
   const uint32_t f_new = (uint32_t)(packed >> 32), ef_new = (uint32_t)packed;
@@ -251,7 +289,9 @@ __device__ void ms_finish(MsState *st, unsigned long long cond, int use_cond) {
   st->lvl = lvl;
   st->next_packed = 0;
   st->done_blocks = 0;
-  st->launches += 3;  // explore, levelgen, expand check
+  st->full = ms_full_classes(st);
+  st->not_full = 0;
+  st->launches += 3;  // explore, classes and expand check, levelgen
   if (f_new > 0 && lvl >= st->level_cap) {
     st->error |= BFS_DEVERR_LEVEL_LIMIT;
     st->F = 0;
@@ -264,7 +304,12 @@ __device__ void ms_finish(MsState *st, unsigned long long cond, int use_cond) {
 // below kHistLevels are recorded as masks, hist[L][v] = new (written for
 // every vertex, coalesced; ms_expand_kernel turns them into the level rows);
 // deeper levels are written straight into the rows.  Kept vertices are
-// compacted with ballot/popc and one atomic per block.
+// compacted with ballot/popc and one atomic per block.  (Eight groups of 32
+// vertices per warp with one atomic per warp and no block barrier: 95 us per
+// large level of R-MAT scale 22 instead of 70; and the 3 blocks per SM it
+// leaves room for reserve slots from three times as wide a window of ids, which
+// scatters the queue and with it the next level's probes: explore's largest
+// level of scale 25 8.4 -> 10.4 ms.)
 __global__ void __launch_bounds__(kMsBlock) ms_levelgen_kernel(MsState *__restrict__ st,
                                                                unsigned long long cond,
                                                                int use_cond) {
@@ -293,6 +338,8 @@ __global__ void __launch_bounds__(kMsBlock) ms_levelgen_kernel(MsState *__restri
   const uint32_t hub_words = st->hub_words;
   const uint32_t *__restrict__ perm = st->perm;
   const uint32_t *__restrict__ moved = st->moved;
+  const uint32_t full = ms_full_classes(st);
+  const uint32_t *__restrict__ skip = full ? st->skip[full - 1u] : nullptr;
   if (threadIdx.x == 0) s_any = 0;
   __syncthreads();
   bool any = false;
@@ -311,6 +358,7 @@ __global__ void __launch_bounds__(kMsBlock) ms_levelgen_kernel(MsState *__restri
         if (v < n_rows) {
           b = indptr[v];
           e = indptr[v + 1];
+          if (skip) b += skip[v];
         }
       }
       if (hist) hist[v] = nw;
@@ -375,21 +423,46 @@ __global__ void __launch_bounds__(kMsBlock) ms_levelgen_kernel(MsState *__restri
   }
 }
 
-// Writes the level rows from the history and, after the last level, the
-// per-root edge counts.  In the level loop (final == 0) it acts only once,
-// right after the last history level when the search goes on: it then
-// writes every row entry (level or -1) so that level generation can write
-// the deeper levels directly.  After the loop (final != 0) it writes the rows
-// unless that already happened (the search went past the history), then
-// adds, per root, the degrees of the vertices < n_rows it reached
+// Between explore and level generation: which further target classes every
+// root has reached to the last vertex.  The grid looks at the classes'
+// vertices together; a block stops after a class that some block has found
+// wanting.
+__device__ __forceinline__ void ms_between_classes(MsState *st) {
+  const unsigned long long all_roots =
+      st->n_lanes >= 64u ? ~0ull : (1ull << st->n_lanes) - 1ull;
+  const uint32_t tid = blockIdx.x * kMsBlock + threadIdx.x, stride = gridDim.x * kMsBlock;
+  for (uint32_t c = st->full; c < st->skip_classes; c++) {
+    const uint32_t v0 = c ? st->skip_limit[c - 1u] : 0u, v1 = st->skip_limit[c];
+    bool all = true;
+    for (uint32_t v = v0 + tid; v < v1; v += stride) all &= st->vis[v] == all_roots;
+    if (!__syncthreads_and(all)) {
+      if (threadIdx.x == 0) atomicOr(&st->not_full, 1u << c);
+      return;
+    }
+    // a class above c found wanting says nothing about the ones between
+    const uint32_t nf = *(volatile uint32_t *)&st->not_full & ((2u << c) - 1u);
+    if (__syncthreads_or(nf != 0u)) return;
+  }
+}
+
+// In the level loop (final == 0, between explore and level generation): looks
+// for classes reached by every root and, when the next level is the first past
+// the history, writes every row entry (level or -1) so that level generation
+// can write the deeper levels directly.  After the loop (final != 0) it writes
+// the rows unless that already happened (the search went past the history),
+// then adds, per root, the degrees of the vertices < n_rows it reached
 // (run_bfs_cpu.hpp:36).
 //
-// One warp per 32 consecutive vertices, lane = vertex.  History levels are
-// < 16, so a lane ORs its vertex's masks into four bit planes (plane k holds
-// the roots whose level has bit k set) and a reached mask; the level of root
-// j is then four bit extracts, and the warp stores root j's 32 entries as one
-// 128-byte segment.  The root loop is unrolled so that every shift is a
-// constant.
+// Rows: one warp per 128 consecutive vertices and 32 roots, four vertices per
+// lane.  History levels are < 16, so a lane ORs its vertices' masks into four
+// bit planes (plane k holds the roots whose level has bit k set) and a reached
+// mask; the level of root j is then four bit extracts, and the warp stores root
+// j's 128 entries as four 128-byte segments in a row.  Bound by the row
+// stores (R-MAT scale 22, 64 roots: 1.07 GB in 0.40 of the kernel's 0.56 ms;
+// 0.61 ms with one vertex per lane and all 64 roots per warp; ER 1 M vertices
+// 254 -> 175 us).  One, two or eight vertices per lane, and rows of 32 roots
+// at a time over the whole range of vertices, were slower; streaming stores
+// save 1 % of a pass.
 // Spreads the 4 low bits of n (n < 16) to bit 0 of the 4 bytes: the shifted
 // copies n, n << 7, n << 14, n << 21 do not overlap, so the product has no
 // carries and byte i holds bit i of n.
@@ -406,136 +479,159 @@ __device__ __forceinline__ int32_t sext_byte(uint32_t x, int i) {
   return (int32_t)r;
 }
 
-template <int H>
-__device__ __forceinline__ void ms_store_rows(int32_t *__restrict__ row, size_t n, uint32_t v,
-                                              bool in, uint32_t nl, uint32_t r, uint32_t b0,
-                                              uint32_t b1, uint32_t b2, uint32_t b3) {
+// Stores the rows of up to 32 roots (nl of them, `row` the first) for the
+// vertices v + 32 i (i < kXv) of a warp's lanes: kXv 128-byte segments of a row
+// follow each other.
+constexpr int kXv = 4;
+constexpr int kXl = 4;  // history levels loaded together
+constexpr int kXb = 3;  // blocks per SM
+__device__ __forceinline__ void ms_store_rows(int32_t *__restrict__ row, size_t n, uint64_t v,
+                                              uint32_t nl, const uint32_t (&r)[kXv],
+                                              const uint32_t (&b0)[kXv], const uint32_t (&b1)[kXv],
+                                              const uint32_t (&b2)[kXv], const uint32_t (&b3)[kXv]) {
   // four roots at a time: their levels as four bytes (0xFF = unreached)
-#pragma unroll
+#pragma unroll 2
   for (int j = 0; j < 32; j += 4) {
-    if ((uint32_t)(H * 32 + j) >= nl) break;  // uniform
-    const uint32_t lv4 = nibble_to_bytes((b0 >> j) & 15u) | (nibble_to_bytes((b1 >> j) & 15u) << 1) |
-                         (nibble_to_bytes((b2 >> j) & 15u) << 2) |
-                         (nibble_to_bytes((b3 >> j) & 15u) << 3);
-    const uint32_t seen = nibble_to_bytes((r >> j) & 15u) * 0xFFu;
-    const uint32_t packed = lv4 | ~seen;
+    if ((uint32_t)j >= nl) break;  // uniform
+    uint32_t packed[kXv];
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      if ((uint32_t)(H * 32 + j + i) >= nl) break;  // uniform
-      if (in) row[v] = sext_byte(packed, i);
+    for (int i = 0; i < kXv; i++) {
+      const uint32_t lv4 = nibble_to_bytes((b0[i] >> j) & 15u) |
+                           (nibble_to_bytes((b1[i] >> j) & 15u) << 1) |
+                           (nibble_to_bytes((b2[i] >> j) & 15u) << 2) |
+                           (nibble_to_bytes((b3[i] >> j) & 15u) << 3);
+      packed[i] = lv4 | ~(nibble_to_bytes((r[i] >> j) & 15u) * 0xFFu);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      if ((uint32_t)(j + q) >= nl) break;  // uniform
+#pragma unroll
+      for (int i = 0; i < kXv; i++)
+        if (v + 32u * i < n) __stcs(row + v + 32u * i, sext_byte(packed[i], q));
       row += n;
     }
   }
 }
 
-__global__ void __launch_bounds__(kMsBlock, 4) ms_expand_kernel(MsState *__restrict__ st,
+__global__ void __launch_bounds__(kMsBlock, kXb) ms_expand_kernel(MsState *__restrict__ st,
                                                                 int final) {
   static_assert(kHistLevels <= 16, "levels must fit four bit planes");
   __shared__ unsigned long long s_edges[kLanes];
   __shared__ unsigned long long s_common;
   const uint32_t lvl = st->lvl;
-  const bool expand = final ? (lvl < kHistLevels) : (lvl + 1u == kHistLevels && st->F > 0);
-  if (!final && !expand) return;  // uniform over the grid
-  const uint32_t n = st->n_cols, n_rows = st->n_rows, nl = st->n_lanes;
+  const bool expand = final ? (lvl < kHistLevels) : (lvl + 1u == kHistLevels);
+  if (!final) {
+    if (st->skip_classes) ms_between_classes(st);
+    if (!expand) return;  // uniform over the grid
+  }
+  const uint32_t n_rows = st->n_rows, nl = st->n_lanes;
+  const uint64_t n = st->n_cols;
   const uint32_t lmax = lvl < kHistLevels ? lvl : kHistLevels - 1u;
-  const unsigned long long *__restrict__ hist = st->hist;
-  const unsigned long long *__restrict__ vis = st->vis;
   const uint32_t *__restrict__ indptr = st->indptr;
   int32_t *__restrict__ level = st->level;
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  if (final) {
-    if (threadIdx.x < kLanes) s_edges[threadIdx.x] = 0;
-    if (threadIdx.x == 0) s_common = 0;
-    __syncthreads();
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t *__restrict__ pinv = st->pinv;
+  const uint32_t *__restrict__ moved = st->moved;
+  const uint64_t gwarp = ((uint64_t)blockIdx.x * kMsBlock + threadIdx.x) >> 5;
+  const uint64_t warps = (uint64_t)gridDim.x * (kMsBlock / 32);
+  if (expand) {
+    // an item: 32 kXv vertices and 32 roots (one half of the masks)
+    const uint32_t halves = nl > 32u ? 2u : 1u;
+    const uint32_t *__restrict__ hist = reinterpret_cast<const uint32_t *>(st->hist);
+    const uint64_t items = (n + 32u * kXv - 1u) / (32u * kXv) * halves;
+    for (uint64_t it = gwarp; it < items; it += warps) {
+      const uint32_t half = halves == 2u ? (uint32_t)it & 1u : 0u;
+      const uint64_t ov = it / halves * (32u * kXv) + lane;  // original ids ov + 32 i
+      uint32_t r[kXv], p0[kXv], p1[kXv], p2[kXv], p3[kXv];
+      const uint32_t *at[kXv];
+#pragma unroll
+      for (int i = 0; i < kXv; i++) {
+        const uint64_t o = ov + 32u * i;
+        // internal id whose masks belong to it (moved ids only differ)
+        uint64_t v = o;
+        if (moved && o < n && ((moved[o >> 5] >> (o & 31u)) & 1u)) v = pinv[o];
+        at[i] = hist + 2u * v + half;
+        r[i] = p0[i] = p1[i] = p2[i] = p3[i] = 0u;
+      }
+      // within levels L0 .. L0 + 3 (L0 a multiple of 4) bits 0 and 1 of the
+      // level are those of k, bits 2 and 3 those of L0
+      for (uint32_t L0 = 0; L0 <= lmax; L0 += kXl) {
+        uint32_t m[kXl][kXv];
+#pragma unroll
+        for (int k = 0; k < kXl; k++)
+#pragma unroll
+          for (int i = 0; i < kXv; i++)
+            m[k][i] = (L0 + k <= lmax && ov + 32u * i < n)
+                          ? at[i][(size_t)(L0 + k) * 2u * n] : 0u;
+#pragma unroll
+        for (int i = 0; i < kXv; i++) {
+#pragma unroll
+          for (int h = 0; h < kXl; h += 4) {
+            const uint32_t all4 = m[h][i] | m[h + 1][i] | m[h + 2][i] | m[h + 3][i];
+            r[i] |= all4;
+            p0[i] |= m[h + 1][i] | m[h + 3][i];
+            p1[i] |= m[h + 2][i] | m[h + 3][i];
+            if ((L0 + h) & 4u) p2[i] |= all4;
+            if ((L0 + h) & 8u) p3[i] |= all4;
+          }
+        }
+      }
+      ms_store_rows(level + (size_t)(half * 32u) * n, n, ov, min(32u, nl - half * 32u), r, p0, p1,
+                    p2, p3);
+    }
   }
+  if (!final) return;
+  if (threadIdx.x < kLanes) s_edges[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_common = 0;
+  __syncthreads();
+  const unsigned long long *__restrict__ vis = st->vis;
   const unsigned long long all_roots = nl >= 64u ? ~0ull : (1ull << nl) - 1ull;
   unsigned long long acc_lo = 0, acc_hi = 0;  // degree sums of roots lane, 32 + lane
   unsigned long long common = 0;              // degree sums of vertices every root reached
-  const uint64_t stride = (uint64_t)gridDim.x * kMsBlock;
-  const uint32_t *__restrict__ pinv = st->pinv;
-  const uint32_t *__restrict__ moved = st->moved;
-  for (uint64_t t0 = (uint64_t)blockIdx.x * kMsBlock + warp * 32u; t0 < n; t0 += stride) {
-    const uint32_t ov = (uint32_t)t0 + lane;  // original id: the row entry written
-    const bool in = ov < n;
-    // internal id whose masks and degree belong to it (moved ids only differ)
-    const uint32_t v = (in && moved && ((moved[ov >> 5] >> (ov & 31u)) & 1u)) ? pinv[ov] : ov;
-    // this step's loads are issued together: the mask and degree for the
-    // edge counts, and history levels 0 .. 7 (8 .. 15 after them, if the
-    // search went that deep)
+  for (uint64_t t0 = gwarp * 32u; t0 < n_rows; t0 += warps * 32u) {  // internal ids
+    const uint64_t v = t0 + lane;
     unsigned long long vm = 0;
     uint32_t d = 0;
-    if (final && in) {
+    if (v < n_rows) {
       vm = vis[v];
-      if (v < n_rows) d = indptr[v + 1] - indptr[v];
+      d = indptr[v + 1] - indptr[v];
     }
-    if (expand) {
-      unsigned long long r = 0, p0 = 0, p1 = 0, p2 = 0, p3 = 0;
-      if (in) {
-        // within levels L0 .. L0 + 3 (L0 a multiple of 4) bits 0 and 1 of
-        // the level are those of k, bits 2 and 3 those of L0
-        for (uint32_t L0 = 0; L0 <= lmax; L0 += 8) {
-          unsigned long long m[8];
+    // per-root degree sums as a bit-matrix product: lane j takes the vertex
+    // masks of roots j and 32 + j (32 ballots), and the degrees go in bit
+    // planes (one ballot per degree bit)
+    const uint32_t deg = vm ? d : 0u;
+    const uint32_t dmax = __reduce_max_sync(kFull, deg);
+    // the usual warp: every vertex with edges was reached by every root
+    // (the giant component), so its degrees count once for all roots
+    if (dmax && __all_sync(kFull, deg == 0u || vm == all_roots)) {
+      common += __reduce_add_sync(kFull, deg);
+    } else if (dmax) {
+      const uint32_t lo = (uint32_t)vm, hi = (uint32_t)(vm >> 32);
+      uint32_t mlo = 0, mhi = 0;
 #pragma unroll
-          for (int k = 0; k < 8; k++)
-            m[k] = (L0 + k <= lmax) ? hist[(size_t)(L0 + k) * n + v] : 0ull;
-#pragma unroll
-          for (int h = 0; h < 8; h += 4) {
-            const unsigned long long all4 = m[h] | m[h + 1] | m[h + 2] | m[h + 3];
-            r |= all4;
-            p0 |= m[h + 1] | m[h + 3];
-            p1 |= m[h + 2] | m[h + 3];
-            if ((L0 + h) & 4u) p2 |= all4;
-            if ((L0 + h) & 8u) p3 |= all4;
-          }
+      for (int j = 0; j < 32; j++) {
+        const uint32_t a = __ballot_sync(kFull, (lo >> j) & 1u);
+        const uint32_t c = __ballot_sync(kFull, (hi >> j) & 1u);
+        if (lane == (uint32_t)j) {
+          mlo = a;
+          mhi = c;
         }
       }
-      ms_store_rows<0>(level, n, ov, in, nl, (uint32_t)r, (uint32_t)p0, (uint32_t)p1,
-                       (uint32_t)p2, (uint32_t)p3);
-      if (nl > 32)
-        ms_store_rows<1>(level + (size_t)32 * n, n, ov, in, nl, (uint32_t)(r >> 32),
-                         (uint32_t)(p0 >> 32), (uint32_t)(p1 >> 32), (uint32_t)(p2 >> 32),
-                         (uint32_t)(p3 >> 32));
-    }
-    if (final) {
-      // per-root degree sums as a bit-matrix product: lane j takes the
-      // vertex masks of roots j and 32 + j (32 ballots), and the degrees go
-      // in bit planes (one ballot per degree bit)
-      const uint32_t deg = vm ? d : 0u;
-      const uint32_t dmax = __reduce_max_sync(kFull, deg);
-      // the usual warp: every vertex with edges was reached by every root
-      // (the giant component), so its degrees count once for all roots
-      if (dmax && __all_sync(kFull, deg == 0u || vm == all_roots)) {
-        common += __reduce_add_sync(kFull, deg);
-      } else if (dmax) {
-        const uint32_t lo = (uint32_t)vm, hi = (uint32_t)(vm >> 32);
-        uint32_t mlo = 0, mhi = 0;
-#pragma unroll
-        for (int j = 0; j < 32; j++) {
-          const uint32_t a = __ballot_sync(kFull, (lo >> j) & 1u);
-          const uint32_t c = __ballot_sync(kFull, (hi >> j) & 1u);
-          if (lane == (uint32_t)j) {
-            mlo = a;
-            mhi = c;
-          }
-        }
-        const int nbits = 32 - __clz(dmax);
-        for (int b = 0; b < nbits; b++) {
-          const uint32_t plane = __ballot_sync(kFull, (deg >> b) & 1u);
-          acc_lo += (unsigned long long)__popc(mlo & plane) << b;
-          acc_hi += (unsigned long long)__popc(mhi & plane) << b;
-        }
+      const int nbits = 32 - __clz(dmax);
+      for (int b = 0; b < nbits; b++) {
+        const uint32_t plane = __ballot_sync(kFull, (deg >> b) & 1u);
+        acc_lo += (unsigned long long)__popc(mlo & plane) << b;
+        acc_hi += (unsigned long long)__popc(mhi & plane) << b;
       }
     }
   }
-  if (final) {
-    if (acc_lo) atomicAdd(&s_edges[lane], acc_lo);
-    if (acc_hi) atomicAdd(&s_edges[32 + lane], acc_hi);
-    if (lane == 0 && common) atomicAdd(&s_common, common);
-    __syncthreads();
-    if (threadIdx.x < nl && s_edges[threadIdx.x] + s_common)
-      atomicAdd(&st->edges[threadIdx.x], s_edges[threadIdx.x] + s_common);
-    if (blockIdx.x == 0 && threadIdx.x == 0) st->launches += 1;
-  }
+  if (acc_lo) atomicAdd(&s_edges[lane], acc_lo);
+  if (acc_hi) atomicAdd(&s_edges[32 + lane], acc_hi);
+  if (lane == 0 && common) atomicAdd(&s_common, common);
+  __syncthreads();
+  if (threadIdx.x < nl && s_edges[threadIdx.x] + s_common)
+    atomicAdd(&st->edges[threadIdx.x], s_edges[threadIdx.x] + s_common);
+  if (blockIdx.x == 0 && threadIdx.x == 0) st->launches += 1;
 }
 
 }  // namespace bfsgb
@@ -625,6 +721,11 @@ static bfs_status ms_setup(bfs_graph *g) {
     s.moved = g->hub->moved;
     s.hubfull = w->hubfull;
     s.hub_words = ms_hub / 32u;
+    s.skip_classes = g->hub->classes;
+    for (uint32_t c = 0; c < g->hub->classes; c++) {
+      s.skip[c] = g->hub->skip[c];
+      s.skip_limit[c] = g->hub->limit[c];
+    }
     s.hub_min_edges = g->hub_min_edges ? g->hub_min_edges
                                        : std::max<uint32_t>(kHubMinEdges, 2u * ms_hub);
     if (hub_bytes > 48 * 1024)
@@ -653,7 +754,7 @@ static bfs_status ms_setup(bfs_graph *g) {
   w->grid_xp = g->num_sms * std::max(occ_xp, 1);
 
   // graph: memset(vis, prev, hist[0]) -> init ->
-  //   while(F > 0) { explore -> levelgen -> expand(in loop) } -> expand(final)
+  //   while(F > 0) { explore -> classes, expand(in loop) -> levelgen } -> expand(final)
   MK(cudaGraphCreate(&w->graph, 0));
   cudaGraphConditionalHandle cond;
   MK(cudaGraphConditionalHandleCreate(&cond, w->graph, 0, cudaGraphCondAssignDefault));
@@ -702,18 +803,20 @@ static bfs_status ms_setup(bfs_graph *g) {
   kp.kernelParams = ex_args;
   MK(cudaGraphAddKernelNode(&n_ex, body, nullptr, 0, &kp));
   kp.sharedMemBytes = 0;
-  void *lg_args[] = {&st, &cond_arg, &one};
-  kp.func = (void *)ms_levelgen_kernel;
-  kp.gridDim = dim3(w->grid_lg);
-  kp.blockDim = dim3(kMsBlock);
-  kp.kernelParams = lg_args;
-  MK(cudaGraphAddKernelNode(&n_lg, body, &n_ex, 1, &kp));
   int in_loop = 0, after = 1;
   void *xp_args[] = {&st, &in_loop};
   kp.func = (void *)ms_expand_kernel;
   kp.gridDim = dim3(w->grid_xp);
+  kp.blockDim = dim3(kMsBlock);
   kp.kernelParams = xp_args;
-  MK(cudaGraphAddKernelNode(&n_xp, body, &n_lg, 1, &kp));
+  MK(cudaGraphAddKernelNode(&n_xp, body, &n_ex, 1, &kp));
+  void *lg_args[] = {&st, &cond_arg, &one};
+  kp.func = (void *)ms_levelgen_kernel;
+  kp.gridDim = dim3(w->grid_lg);
+  kp.kernelParams = lg_args;
+  MK(cudaGraphAddKernelNode(&n_lg, body, &n_xp, 1, &kp));
+  kp.func = (void *)ms_expand_kernel;
+  kp.gridDim = dim3(w->grid_xp);
   void *xf_args[] = {&st, &after};
   kp.kernelParams = xf_args;
   MK(cudaGraphAddKernelNode(&n_xf, w->graph, &n_while, 1, &kp));
@@ -740,9 +843,9 @@ static bfs_status ms_pass_host(bfs_graph *g, MsWorkspace *w) {
     if (*h_F == 0) break;
     ms_explore_kernel<<<w->grid_ex, kMsBlock, w->hub_bytes, s>>>(st);
     MK(cudaGetLastError());
-    ms_levelgen_kernel<<<w->grid_lg, kMsBlock, 0, s>>>(st, no_cond, zero);
-    MK(cudaGetLastError());
     ms_expand_kernel<<<w->grid_xp, kMsBlock, 0, s>>>(st, 0);
+    MK(cudaGetLastError());
+    ms_levelgen_kernel<<<w->grid_lg, kMsBlock, 0, s>>>(st, no_cond, zero);
     MK(cudaGetLastError());
   }
   ms_expand_kernel<<<w->grid_xp, kMsBlock, 0, s>>>(st, 1);

@@ -73,3 +73,22 @@ def test_levels_with_classes_left_out(B, O, n, K, symmetric):
                     tab = st.levels_table()
                     assert sum(tab["edges"]) == ec
     dg.free()
+
+
+@pytest.mark.parametrize("symmetric", [False, True])
+@pytest.mark.parametrize("n,K", [(2047, 128), (20011, 128), (70001, 4096)])
+def test_batches_with_classes_left_out(B, O, n, K, symmetric):
+    """Batched runs: a class is left out once all roots of the pass (64, and 6
+    in the last) have reached it; depths past the 16 levels of history."""
+    torch = torch_cuda()
+    g = skewed(B, n, 12 * n, [255, 257, 9001], n, symmetric)
+    dg = B.Graph.upload(g)
+    dg.hub_configure(K, min_edges=1)
+    roots = B.sample_roots(g, 70, n)
+    roots[3] = roots[9]
+    ref, rec = O.oracle_bfs_many(g.indptr, g.inds, roots, queue_form=True)
+    out = torch.full((len(roots), n), 7, dtype=torch.int32, device="cuda")
+    for loop in ("graph", "host"):
+        ec, _ = dg.run_batch(roots, out.data_ptr(), loop=loop)
+        assert np.array_equal(out.cpu().numpy(), ref) and np.array_equal(ec, rec), loop
+    dg.free()
