@@ -12,7 +12,8 @@
 // warps, owners resolved per warp round (bfs_internal / device_util), IPT
 // rounds in flight per lane.  A claim is an atomicOr on the shared bitmap; the
 // claiming thread writes the level and appends the vertex to the next queue
-// (vertices >= n_rows or without out-edges get a level but are not queued).
+// (vertices >= n_rows get a level but are not queued; those without out-edges
+// are dropped when the next level loads their offsets).
 //
 // Block size (128/256/512) and items per thread (1/2/4 rounds per lane) come
 // from an autotuner that times every combination on the batch and caches the
@@ -65,25 +66,49 @@ struct MultiArgs {
   unsigned long long *edges_out;
 };
 
+// Shared memory of a block beside its bitmap.
+template <int B>
+struct MultiTile {
+  uint32_t off[B + 1];  // first round unit (edge or chunk) of an entry, in the tile
+  uint32_t beg[B];      // first edge
+  uint32_t deg[B];
+  uint2 wsum[B / 32];
+  uint32_t next, graph;
+};
+
 // One level of one graph over tiles tile0, tile0 + tstride, ... of B
-// frontier entries (LLB form): block exclusive scan of the tile's degrees,
-// the tile's edges split evenly over the warps, owners resolved per warp
-// round, IPT rounds in flight per lane.  A claim is an atomicOr on the
-// visited bitmap -- the block's own shared bitmap, or, for a graph shared by
-// a cluster (CL), the cluster's bitmap in global memory, with the shared
-// bitmap kept as a filter of already visited vertices.  The claiming thread
-// writes the level; kept vertices are appended to qn through *ctr (a shared
-// counter per vertex, or for CL a global counter per warp round).  Returns
-// (in thread 0) the sum of the tiles' degrees.
+// frontier entries (LLB form): block exclusive scan over the tile, entries
+// without edges dropped, the tile's edges split evenly over the warps, owners
+// resolved per warp round.  With IPT = 4 a round deals 16-byte chunks of the
+// edge array, one per lane -- four edges in flight for one owner resolution;
+// otherwise IPT rounds of single edges.  A claim is an atomicOr on the visited
+// bitmap -- the block's own shared bitmap, or, for a graph shared by a cluster
+// (CL), the cluster's bitmap in global memory, with the shared bitmap kept as a
+// filter of already visited vertices; a lane's claims are in flight together.
+// The claiming thread writes the level; the warp's new vertices are appended to
+// qn through one atomic on *ctr (shared, or global for CL).  Their degrees are
+// not looked at here, so no dependent load waits in the innermost loop.
+// Returns this thread's part of the sum of the tiles' degrees.  Bound by
+// instruction issue on the busiest SMs; 256 R-MAT graphs of scales 10-16, best
+// configuration 1.10 -> 0.59 ms: without the degree look-up and one-by-one
+// appends, and with the cluster's filter copied from its bitmap instead of
+// merged from a long frontier, 1.10 -> 0.93; a quarter of a cluster's fair share
+// instead of a whole one as the limit for sharing a graph 0.93 -> 0.78 (half,
+// eighth, sixteenth: 0.79, 0.78, 0.81); chunks 0.78 -> 0.59.  Registers for 2
+// or 3 blocks of 512 threads per SM instead of 4: 0.80, 0.76.
 template <int B, int IPT, bool CL>
 __device__ __forceinline__ unsigned long long multi_level(
     const uint32_t *__restrict__ ip, const uint32_t *__restrict__ ix, int32_t *lv,
     uint32_t n_rows, const uint32_t *qc, uint32_t *qn, uint32_t F, int32_t lvl,
     uint32_t tile0, uint32_t tstride, uint32_t *s_bitmap, uint32_t *gb, uint32_t *ctr,
-    uint32_t *s_off, uint32_t *s_beg, uint32_t *s_wsum) {
+    MultiTile<B> &s) {
   constexpr int NW = B / 32;
+  constexpr bool kChunks = IPT == 4;
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t lt_mask = (1u << lane) - 1u;
+  // chunks are counted from the 16-byte boundary at or below ix
+  const uint32_t eoff = kChunks ? (uint32_t)((reinterpret_cast<uintptr_t>(ix) & 15u) >> 2) : 0u;
+  const uint4 *__restrict__ ix4 = reinterpret_cast<const uint4 *>(ix - eoff);
   unsigned long long edges = 0;
   for (uint32_t tile = tile0; tile < F; tile += tstride) {
     const uint32_t slot = tile + threadIdx.x;
@@ -92,97 +117,126 @@ __device__ __forceinline__ unsigned long long multi_level(
       const uint32_t u = CL ? __ldcg(qc + slot) : qc[slot];
       beg = ip[u];
       deg = ip[u + 1] - beg;
+      beg += eoff;
     }
-    const uint32_t incl = warp_incl_scan(deg, lane);
-    if (lane == 31) s_wsum[warp] = incl;
+    edges += deg;
+    const uint32_t units = kChunks ? edge_chunks(beg, deg, 0u) : deg;
+    const uint32_t incl = warp_incl_scan(units, lane);
+    const uint32_t has = __ballot_sync(kFull, deg > 0u);
+    if (lane == 31) s.wsum[warp] = make_uint2(incl, __popc(has));
     __syncthreads();
-    if (warp == 0) {
-      uint32_t w = lane < (uint32_t)NW ? s_wsum[lane] : 0u;
-      w = warp_incl_scan(w, lane);
-      if (lane < (uint32_t)NW) s_wsum[lane] = w;
+    const uint2 ws = lane < (uint32_t)NW ? s.wsum[lane] : make_uint2(0u, 0u);
+    const uint32_t wu = warp_incl_scan(ws.x, lane), wc = warp_incl_scan(ws.y, lane);
+    const uint32_t total = __shfl_sync(kFull, wu, 31), m = __shfl_sync(kFull, wc, 31);
+    const uint32_t uprev = __shfl_sync(kFull, wu, (warp + 31u) & 31u);
+    const uint32_t cprev = __shfl_sync(kFull, wc, (warp + 31u) & 31u);
+    if (deg) {
+      const uint32_t i = (warp ? cprev : 0u) + __popc(has & lt_mask);
+      s.off[i] = (warp ? uprev : 0u) + incl - units;
+      s.beg[i] = beg;
+      if (kChunks) s.deg[i] = deg;
     }
-    __syncthreads();
-    const uint32_t total = s_wsum[NW - 1];
-    s_off[threadIdx.x] = (warp ? s_wsum[warp - 1] : 0u) + incl - deg;
-    s_beg[threadIdx.x] = beg;
-    if (threadIdx.x == 0) s_off[B] = total;
+    if (threadIdx.x == 0) s.off[m] = total;
     __syncthreads();
     const uint32_t per_warp = ((total + NW - 1) / NW + 31u) & ~31u;
     const uint32_t w0 = warp * per_warp;
     if (w0 < total) {
       const uint32_t w1 = min(total, w0 + per_warp);
-      uint32_t lo = 0, hi = B;
+      uint32_t lo = 0, hi = m;
       while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (s_off[mid] <= w0) lo = mid; else hi = mid;
+        if (s.off[mid] <= w0) lo = mid; else hi = mid;
       }
       uint32_t cur = lo;
-      for (uint32_t base = w0; base < w1; base += 32u * IPT) {
-        uint32_t addr[IPT];
-#pragma unroll
-        for (int u = 0; u < IPT; u++) {
-          const uint32_t rb = base + 32u * u;
-          const uint32_t e = rb + lane;
+      for (uint32_t base = w0; base < w1; base += kChunks ? 32u : 32u * IPT) {
+        uint32_t nb[IPT], on = 0;  // targets; bit u: slot u holds one
+        if constexpr (kChunks) {
+          const uint32_t x = base + lane;
           const uint32_t j = cur + 1u + lane;
-          const uint32_t bnd = (j <= (uint32_t)B) ? s_off[j] : kFull;
-          const uint32_t p = bnd - rb;
-          const uint32_t starts = __reduce_or_sync(kFull, (p < 32u) ? (1u << p) : 0u);
-          const uint32_t o = cur + __popc(starts & ((2u << lane) - 1u));
-          addr[u] = (e < w1) ? s_beg[o] + (e - s_off[o]) : kFull;
-          cur = __shfl_sync(kFull, o, 31);
-          if (cur >= (uint32_t)B) cur = B - 1;
-        }
-        uint32_t nb[IPT];
+          const uint32_t bnd = j <= m ? s.off[j] : kFull;
+          const uint32_t starts = __reduce_or_sync(kFull, bit_or_zero(bnd - base));
+          uint32_t o = cur + __popc(starts & ((2u << lane) - 1u));
+          cur += __popc(starts);
+          if (cur >= m) cur = m - 1;  // only reached past w1
+          if (o >= m) o = m - 1;
+          const uint32_t sb = s.beg[o], sd = s.deg[o];
+          const uint32_t a4 = (sb >> 2) + (x - s.off[o]), p0 = a4 << 2;
+          uint4 q = make_uint4(0u, 0u, 0u, 0u);
+          if (x < w1) {
+            const uint32_t from = sb > p0 ? sb - p0 : 0u, left = sb + sd - p0;
+            on = (0xFu >> (4u - (left < 4u ? left : 4u))) & (0xFu << from);
+            q = __ldg(ix4 + a4);  // the packed array is padded to whole chunks
+          }
+          nb[0] = q.x;
+          nb[1] = q.y;
+          nb[2] = q.z;
+          nb[3] = q.w;
+        } else {
+          uint32_t addr[IPT];
 #pragma unroll
-        for (int u = 0; u < IPT; u++) nb[u] = addr[u] != kFull ? ix[addr[u]] : 0u;
+          for (int u = 0; u < IPT; u++) {
+            const uint32_t rb = base + 32u * u;
+            const uint32_t e = rb + lane;
+            const uint32_t j = cur + 1u + lane;
+            const uint32_t bnd = j <= m ? s.off[j] : kFull;
+            const uint32_t starts = __reduce_or_sync(kFull, bit_or_zero(bnd - rb));
+            const uint32_t o = cur + __popc(starts & ((2u << lane) - 1u));
+            addr[u] = (e < w1) ? s.beg[o] + (e - s.off[o]) : kFull;
+            cur += __popc(starts);
+            if (cur >= m) cur = m - 1;  // only reached past w1
+          }
+#pragma unroll
+          for (int u = 0; u < IPT; u++) {
+            nb[u] = addr[u] != kFull ? ix[addr[u]] : 0u;
+            on |= addr[u] != kFull ? 1u << u : 0u;
+          }
+        }
+        uint32_t old[IPT];
 #pragma unroll
         for (int u = 0; u < IPT; u++) {
-          bool push = false;
-          const uint32_t v = nb[u];
-          if (addr[u] != kFull) {
-            const uint32_t w = v >> 5, bit = 1u << (v & 31u);
-            if (!(s_bitmap[w] & bit)) {
-              uint32_t old;
-              if (CL) {
-                old = atomicOr(gb + w, bit);
-                atomicOr(s_bitmap + w, bit);
-              } else {
-                old = atomicOr(s_bitmap + w, bit);
-              }
-              if (!(old & bit)) {
-                lv[v] = lvl + 1;
-                push = v < n_rows && ip[v + 1] > ip[v];
-                // a block's own queue: one shared-memory atomic per vertex
-                if (!CL && push) qn[atomicAdd(ctr, 1u)] = v;
-              }
-            }
+          const uint32_t w = nb[u] >> 5, bit = 1u << (nb[u] & 31u);
+          old[u] = kFull;  // visited
+          if (((on >> u) & 1u) && !(s_bitmap[w] & bit)) {
+            old[u] = atomicOr((CL ? gb : s_bitmap) + w, bit);
+            if (CL) atomicOr(s_bitmap + w, bit);
           }
-          if (CL) {  // a cluster's queue in global memory: one atomic per warp round
-            const uint32_t pm = __ballot_sync(kFull, push);
-            if (pm) {
-              const uint32_t leader = __ffs(pm) - 1u;
-              uint32_t base0 = 0;
-              if (lane == leader) base0 = atomicAdd(ctr, (uint32_t)__popc(pm));
-              base0 = __shfl_sync(kFull, base0, leader);
-              if (push) qn[base0 + __popc(pm & lt_mask)] = v;
-            }
-          }
+        }
+        uint32_t push[IPT], num = 0;
+#pragma unroll
+        for (int u = 0; u < IPT; u++) {
+          const bool mine = !((old[u] >> (nb[u] & 31u)) & 1u);
+          if (mine) lv[nb[u]] = lvl + 1;
+          push[u] = __ballot_sync(kFull, mine && nb[u] < n_rows);
+          num += __popc(push[u]);
+        }
+        if (num == 0u) continue;  // uniform over the warp
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(ctr, num);
+        at = __shfl_sync(kFull, at, 0);
+#pragma unroll
+        for (int u = 0; u < IPT; u++) {
+          if ((push[u] >> lane) & 1u) qn[at + __popc(push[u] & lt_mask)] = nb[u];
+          at += __popc(push[u]);
         }
       }
     }
-    if (threadIdx.x == 0) edges += total;
     __syncthreads();
   }
   return edges;
+}
+
+// Adds the block's part of a graph's edge count (cleared before the launch).
+__device__ __forceinline__ void add_edges(unsigned long long *out, unsigned long long edges) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) edges += __shfl_xor_sync(kFull, edges, d);
+  if ((threadIdx.x & 31u) == 0 && edges) atomicAdd(out, edges);
 }
 
 // A complete BFS of one graph by one block, the visited bitmap in shared
 // memory and __syncthreads as the level barrier.
 template <int B, int IPT>
 __device__ __forceinline__ void multi_graph_block(const MultiArgs &a, uint32_t gi,
-                                                  uint32_t *s_bitmap, uint32_t *s_off,
-                                                  uint32_t *s_beg, uint32_t *s_wsum,
-                                                  uint32_t *s_next) {
+                                                  uint32_t *s_bitmap, MultiTile<B> &s) {
   const MultiDesc d = a.descs[a.order[gi]];
   const uint32_t *__restrict__ ip = a.indptr_all + d.vbase;
   const uint32_t *__restrict__ ix = a.inds_all + d.ebase;
@@ -198,41 +252,39 @@ __device__ __forceinline__ void multi_graph_block(const MultiArgs &a, uint32_t g
     lv[r] = 0;
     const uint32_t rdeg = r < d.n_rows ? ip[r + 1] - ip[r] : 0u;
     if (rdeg) q0[0] = r;
-    s_next[0] = rdeg ? 1u : 0u;
+    s.next = rdeg ? 1u : 0u;
   }
   __syncthreads();
-  uint32_t F = s_next[0];
+  uint32_t F = s.next;
   uint32_t *qc = q0, *qn = q1;
   unsigned long long edges = 0;
   int32_t lvl = 0;
   while (F > 0) {
     __syncthreads();
-    if (threadIdx.x == 0) s_next[0] = 0;
+    if (threadIdx.x == 0) s.next = 0;
     __syncthreads();
     edges += multi_level<B, IPT, false>(ip, ix, lv, d.n_rows, qc, qn, F, lvl, 0u, B, s_bitmap,
-                                        nullptr, s_next, s_off, s_beg, s_wsum);
+                                        nullptr, &s.next, s);
     __syncthreads();
-    F = s_next[0];
+    F = s.next;
     uint32_t *t = qc;
     qc = qn;
     qn = t;
     lvl++;
   }
-  if (threadIdx.x == 0) a.edges_out[a.order[gi]] = edges;
+  add_edges(a.edges_out + a.order[gi], edges);
 }
 
 // Graphs claimed one per block from a work counter (largest first).
 template <int B, int IPT>
 __device__ __forceinline__ void multi_small_graphs(const MultiArgs &a, uint32_t *s_bitmap,
-                                                   uint32_t *s_off, uint32_t *s_beg,
-                                                   uint32_t *s_wsum, uint32_t *s_next,
-                                                   uint32_t *s_graph) {
+                                                   MultiTile<B> &s) {
   for (;;) {
-    if (threadIdx.x == 0) *s_graph = a.n_big + atomicAdd(&a.work[0], 1u);
+    if (threadIdx.x == 0) s.graph = a.n_big + atomicAdd(&a.work[0], 1u);
     __syncthreads();
-    const uint32_t gi = *s_graph;
+    const uint32_t gi = s.graph;
     if (gi >= a.n_graphs) break;
-    multi_graph_block<B, IPT>(a, gi, s_bitmap, s_off, s_beg, s_wsum, s_next);
+    multi_graph_block<B, IPT>(a, gi, s_bitmap, s);
     __syncthreads();
   }
 }
@@ -240,11 +292,8 @@ __device__ __forceinline__ void multi_small_graphs(const MultiArgs &a, uint32_t 
 template <int B, int IPT>
 __global__ void __launch_bounds__(B, 2048 / B) multi_bfs_kernel(MultiArgs a) {
   extern __shared__ uint32_t s_bitmap[];
-  __shared__ uint32_t s_off[B + 1];
-  __shared__ uint32_t s_beg[B];
-  __shared__ uint32_t s_wsum[B / 32];
-  __shared__ uint32_t s_next[1], s_graph[1];
-  multi_small_graphs<B, IPT>(a, s_bitmap, s_off, s_beg, s_wsum, s_next, s_graph);
+  __shared__ MultiTile<B> s;
+  multi_small_graphs<B, IPT>(a, s_bitmap, s);
 }
 
 // Clusters of C blocks first share the largest graphs (order[0, n_big)): a
@@ -260,10 +309,7 @@ template <int B, int IPT, int C>
 __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(B, 2048 / B)
     multi_bfs_cluster_kernel(MultiArgs a) {
   extern __shared__ uint32_t s_bitmap[];
-  __shared__ uint32_t s_off[B + 1];
-  __shared__ uint32_t s_beg[B];
-  __shared__ uint32_t s_wsum[B / 32];
-  __shared__ uint32_t s_next[1], s_graph[1];
+  __shared__ MultiTile<B> s;
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   const uint32_t rank = cl.block_rank();
@@ -309,22 +355,28 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(B, 2048 / B)
       uint32_t *qn = (lvl & 1) ? cq0 : cq1;
       uint32_t *ctr = cnt + (lvl + 1) % 3;
       edges += multi_level<B, IPT, true>(ip, ix, lv, d.n_rows, qc, qn, F, lvl, rank * B, C * B,
-                                         s_bitmap, gb, ctr, s_off, s_beg, s_wsum);
+                                         s_bitmap, gb, ctr, s);
       cl.sync();
       const uint32_t fn = __ldcg(ctr);
-      // vertices claimed by the other blocks join this block's filter
-      for (uint32_t i = threadIdx.x; i < fn; i += B) {
-        const uint32_t v = __ldcg(qn + i);
-        atomicOr(s_bitmap + (v >> 5), 1u << (v & 31u));
+      // vertices claimed by the other blocks join this block's filter: the
+      // new frontier's, or the whole bitmap where that is shorter
+      if (fn < words) {
+        for (uint32_t i = threadIdx.x; i < fn; i += B) {
+          const uint32_t v = __ldcg(qn + i);
+          atomicOr(s_bitmap + (v >> 5), 1u << (v & 31u));
+        }
+      } else {
+#pragma unroll 4
+        for (uint32_t w = threadIdx.x; w < words; w += B) s_bitmap[w] = __ldcg(gb + w);
       }
       __syncthreads();
       F = fn;
       lvl++;
     }
-    if (threadIdx.x == 0 && edges) atomicAdd(&a.edges_out[a.order[gi]], edges);
+    add_edges(a.edges_out + a.order[gi], edges);
     cl.sync();  // queues, counters and bitmap are free for the cluster's next graph
   }
-  multi_small_graphs<B, IPT>(a, s_bitmap, s_off, s_beg, s_wsum, s_next, s_graph);
+  multi_small_graphs<B, IPT>(a, s_bitmap, s);
 }
 
 __global__ void multi_fill_kernel(int32_t *levels, uint64_t n) {
@@ -420,10 +472,10 @@ static bfs_status multi_prepare(bfs_multi *m, int cfg, int32_t *levels_dev) {
   uint32_t n_big = 0;
   if (c.cluster > 1) {
     grid = std::max(c.cluster, grid / c.cluster * c.cluster);
-    // a graph is shared by a cluster when its edges exceed `cluster` blocks'
-    // fair share of the batch's edges
+    // a graph is shared by a cluster when its edges exceed a quarter of
+    // `cluster` blocks' fair share of the batch's edges
     for (uint32_t i = 0; i < m->n_graphs; i++)
-      if ((double)m->order_nnz[i] * grid >= (double)m->total_edges * c.cluster) n_big = i + 1;
+      if ((double)m->order_nnz[i] * grid * 4.0 >= (double)m->total_edges * c.cluster) n_big = i + 1;
     const size_t n_clusters = (size_t)grid / c.cluster;
     if (m->gbits_words < n_clusters * words) {
       cudaFree(m->d_gbits);
@@ -567,7 +619,8 @@ bfs_status bfs_multi_create(uint32_t n_graphs, const uint32_t *const *indptrs,
   CK2(cudaEventCreate(&m->e0));
   CK2(cudaEventCreate(&m->e1));
   CK2(dev_malloc(&m->d_indptr, sizeof(uint32_t) * vb));
-  CK2(dev_malloc(&m->d_inds, sizeof(uint32_t) * std::max<uint64_t>(eb, 1)));
+  // padded: whole 16-byte chunks of it are read
+  CK2(dev_malloc(&m->d_inds, sizeof(uint32_t) * ((eb + 4) / 4 * 4)));
   CK2(dev_malloc(&m->d_order, sizeof(uint32_t) * n_graphs));
   CK2(dev_malloc(&m->d_work, 2 * sizeof(uint32_t)));
   CK2(dev_malloc(&m->d_descs, sizeof(MultiDesc) * n_graphs));
