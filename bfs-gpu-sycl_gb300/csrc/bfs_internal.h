@@ -170,6 +170,8 @@ struct BfsDevState {
   int32_t *rec_arm;          // arm chosen by a scheduler on the device, -1 if none
   int32_t *rec_ran;          // arm of the explore kernel that ran
   uint32_t rec_cap;
+  BfsDevState *result;       // host copy of the final state (mapped), or null
+  unsigned long long bad;    // CSC errors found by the allocation-free call
 };
 
 enum : uint32_t {

@@ -379,10 +379,10 @@ static cudaError_t add_kernel(cudaGraph_t graph, cudaGraphNode_t *node,
 }
 
 // Builds the device-side level loop:
-//   fill(parents, working levels, bitmaps) -> init(root) -> narrow levels ->
-//   while(F > 0) { explore -> levelgen (last block sets the while condition)
+//   init(root) and narrow levels -> while(F > 0) { explore -> levelgen (last block sets the while condition)
 //                  -> narrow levels (sets it again) } -> level output
-// The narrow-level kernel (narrow.cu) runs consecutive levels of few edges in
+// on a state and workspace that the fill kernel, launched before the graph,
+// has written.  The narrow-level kernel (narrow.cu) seeds the root and runs consecutive levels of few edges in
 // one launch and is left out of recorded runs.
 // With a fixed arm the explore node is that arm's kernel (explore_any for the
 // GLB arms).  With arm < 0 (learned schedule) it is explore_any, which runs
@@ -401,16 +401,16 @@ static bfs_status build_loop_graph(bfs_graph *g, int arm, int sm_factor, int ipt
   int one = 1;
   BfsDevState *st = g->d_st;
 
-  cudaGraphNode_t n_fill, n_init, n_while, n_explore, n_lg;
-  void *fill_args[] = {&st};  // levels (and parents) to -1, bitmaps cleared
-  CK(add_kernel(graph, &n_fill, nullptr, 0, fill_kernel_fn(), g->num_sms * 4, 256, fill_args));
-  void *init_args[] = {&st, &cond_arg, &one};
-  CK(add_kernel(graph, &n_init, &n_fill, 1, init_kernel_fn(), 1, 32, init_args));
+  cudaGraphNode_t n_first, n_while, n_explore, n_lg;
+  void *out_args[] = {&st};
   const void *narrow_fn = narrow ? narrow_kernel_fn(g->narrow_cluster, g->run_parents) : nullptr;
-  cudaGraphNode_t n_narrow = n_init;
+  const size_t narrow_smem = narrow_smem_bytes(g->run_parents);
+  void *init_args[] = {&st, &cond_arg, &one, &one};
   if (narrow)
-    CK(add_kernel(graph, &n_narrow, &n_init, 1, narrow_fn, g->narrow_cluster, kNarrowBlock,
-                  init_args, narrow_smem_bytes(g->run_parents)));
+    CK(add_kernel(graph, &n_first, nullptr, 0, narrow_fn, g->narrow_cluster, kNarrowBlock, init_args,
+                  narrow_smem));
+  else
+    CK(add_kernel(graph, &n_first, nullptr, 0, init_kernel_fn(), 1, 32, init_args));
 
   // cudaGraphNodeParams has no usable default constructor (union members)
   alignas(cudaGraphNodeParams) unsigned char wbuf[sizeof(cudaGraphNodeParams)] = {};
@@ -419,11 +419,11 @@ static bfs_status build_loop_graph(bfs_graph *g, int arm, int sm_factor, int ipt
   wp.conditional.handle = cond;
   wp.conditional.type = cudaGraphCondTypeWhile;
   wp.conditional.size = 1;
-  CK(cudaGraphAddNode(&n_while, graph, &n_narrow, nullptr, 1, &wp));
+  CK(cudaGraphAddNode(&n_while, graph, &n_first, nullptr, 1, &wp));
   cudaGraph_t body = wp.conditional.phGraph_out[0];
   cudaGraphNode_t n_out;
   CK(add_kernel(graph, &n_out, &n_while, 1, level_out_kernel_fn(), g->num_sms * 8, 256,
-                fill_args));
+                out_args));
 
   void *ex_args[] = {&st};
   int arm_arg = arm;  // < 0: the scheduler's arm in st->arm
@@ -443,8 +443,10 @@ static bfs_status build_loop_graph(bfs_graph *g, int arm, int sm_factor, int ipt
   set_window(g, n_lg);
   if (narrow) {
     cudaGraphNode_t n_next;
-    CK(add_kernel(body, &n_next, &n_lg, 1, narrow_fn, g->narrow_cluster, kNarrowBlock, lg_args,
-                  narrow_smem_bytes(g->run_parents)));
+    int zero = 0;
+    void *next_args[] = {&st, &cond_arg, &one, &zero};
+    CK(add_kernel(body, &n_next, &n_lg, 1, narrow_fn, g->narrow_cluster, kNarrowBlock, next_args,
+                  narrow_smem));
   }
   CK(cudaGraphInstantiate(&ge->exec, graph, 0));
   return BFS_OK;
@@ -497,8 +499,7 @@ static bfs_status host_loop(bfs_graph *g, int arm_fixed, int sm_factor, int ipt,
   int zero = 0;
   const bool prof = g->prof_explore != nullptr;
   const bool learned = arm_fixed < 0;
-  void *fill_args[] = {&st};
-  CK(cudaLaunchKernel(fill_kernel_fn(), dim3(g->num_sms * 4), dim3(256), fill_args, 0, g->stream));
+  void *out_args[] = {&st};
   void *init_args[] = {&st, &no_cond, &zero};
   CK(cudaLaunchKernel(init_kernel_fn(), dim3(1), dim3(32), init_args, 0, g->stream));
   uint32_t launches = 2;
@@ -531,7 +532,7 @@ static bfs_status host_loop(bfs_graph *g, int arm_fixed, int sm_factor, int ipt,
     launches += 2;
     if (level < BFS_MAX_RECORDED_LEVELS) g->host_arms[level] = arm;
   }
-  CK(cudaLaunchKernel(level_out_kernel_fn(), dim3(g->num_sms * 8), dim3(256), fill_args, 0,
+  CK(cudaLaunchKernel(level_out_kernel_fn(), dim3(g->num_sms * 8), dim3(256), out_args, 0,
                       g->stream));
   g->host_launches = launches + 1;
   return BFS_OK;
@@ -605,8 +606,7 @@ bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts_
   }
   bfs_status hrc = ensure_hub(g);
   if (hrc != BFS_OK) return hrc;
-  BfsDevState &s = *g->h_st;
-  s = g->tmpl;
+  BfsDevState s = g->tmpl;
   s.root = root;
   s.level = levels_dev;
   s.parent = parents_dev;
@@ -655,7 +655,9 @@ bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts_
     }
   }
   CK(cudaEventRecord(g->ev0, g->stream));
-  CK(launch_seed_state(g->d_st, *g->h_st, g->stream));
+  s.result = graph_loop ? g->h_st : nullptr;  // written by the output pass
+  void *fill_args[] = {&g->d_st, &s};
+  CK(cudaLaunchKernel(fill_kernel_fn(), dim3(g->num_sms * 4), dim3(256), fill_args, 0, g->stream));
   uint32_t launches = 0;
   if (graph_loop) {
     CK(cudaGraphLaunch(ge->exec, g->stream));
@@ -672,8 +674,12 @@ bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts_
       return rc;
     }
   }
-  rc = read_state(g);
-  if (rc != BFS_OK) return rc;
+  if (graph_loop) {
+    CK(cudaStreamSynchronize(g->stream));
+  } else {
+    rc = read_state(g);
+    if (rc != BFS_OK) return rc;
+  }
   const BfsDevState &r = *g->h_st;
   if (r.error & BFS_DEVERR_LEVEL_LIMIT)
     return fail(BFS_ERR_LEVEL_LIMIT, "level loop exceeded n_cols + 1 levels");
@@ -685,7 +691,7 @@ bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts_
     stats->reached = r.reached;
     stats->num_levels = r.max_level + 1;
     stats->device_ms = ms;
-    stats->launches = (launches ? launches : r.launches) + 1;  // + the seed kernel
+    stats->launches = launches ? launches : r.launches;
     stats->recorded = 0;
     if (o.record < 2) {
       std::memset(stats->level_explore_ms, 0, sizeof(stats->level_explore_ms));

@@ -44,6 +44,7 @@
 #include "device_util.cuh"
 #include "kernels.h"
 #include "bfs_sched_dev.cuh"
+#include "level_state.cuh"
 
 namespace bfsgb {
 
@@ -83,9 +84,18 @@ __device__ __forceinline__ uint32_t round_owner(uint32_t cur, uint32_t bnd,
 
 // ---- fill / init --------------------------------------------------------------
 
-__global__ void fill_kernel(BfsDevState *st) {
-  int32_t *parent = st->parent;
-  const uint32_t n = st->n_cols;
+// Also writes the state: the host's template comes by value, so that a BFS
+// uses no copy engine at its start (a copy queued ahead of a run on another
+// stream would hold the run back).
+__global__ void fill_kernel(BfsDevState *st, const BfsDevState s) {
+  static_assert(sizeof(BfsDevState) % 4 == 0, "state is copied in words");
+  if (blockIdx.x == 0) {
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(&s);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(st);
+    for (uint32_t i = threadIdx.x; i < sizeof(BfsDevState) / 4; i += blockDim.x) dst[i] = src[i];
+  }
+  int32_t *parent = s.parent;
+  const uint32_t n = s.n_cols;
   const uint32_t stride = gridDim.x * blockDim.x;
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
   // parents to -1 (int4 stores for the body when the buffer is 16-byte
@@ -96,19 +106,18 @@ __global__ void fill_kernel(BfsDevState *st) {
     for (uint32_t i = tid; i < n4; i += stride) reinterpret_cast<int4 *>(parent)[i] = neg;
     for (uint32_t i = (n4 << 2) + tid; i < n; i += stride) parent[i] = -1;
   }
-  for (uint32_t i = tid; i < st->rec_cap; i += stride) st->rec_ran[i] = -1;
+  for (uint32_t i = tid; i < s.rec_cap; i += stride) s.rec_ran[i] = -1;
   // cleared bitmaps and unvisited working levels: kernel stores rather than
-  // a memset, so that a BFS uses no copy engine between its start and its
-  // final state read (words is a multiple of 32, the bitmaps and the
+  // a memset, for the same reason (words is a multiple of 32, the bitmaps and the
   // working levels -- 32 bytes per word -- are 16-byte aligned)
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  for (uint32_t i = tid; i < (st->words >> 2); i += stride) {
-    reinterpret_cast<uint4 *>(st->vis)[i] = zero;
-    reinterpret_cast<uint4 *>(st->prev)[i] = zero;
+  for (uint32_t i = tid; i < (s.words >> 2); i += stride) {
+    reinterpret_cast<uint4 *>(s.vis)[i] = zero;
+    reinterpret_cast<uint4 *>(s.prev)[i] = zero;
   }
   const uint4 unvisited = make_uint4(~0u, ~0u, ~0u, ~0u);
-  for (uint32_t i = tid; i < st->words * 2u; i += stride)
-    reinterpret_cast<uint4 *>(st->lv8)[i] = unvisited;
+  for (uint32_t i = tid; i < s.words * 2u; i += stride)
+    reinterpret_cast<uint4 *>(s.lv8)[i] = unvisited;
 }
 
 __device__ __forceinline__ int32_t output_level(uint32_t c, const int32_t *level, uint32_t u) {
@@ -126,10 +135,18 @@ __device__ __forceinline__ int4 output_levels4(uint32_t c4, const int32_t *level
 // during the BFS) are kept.  Lane l of a warp step takes the 4-id groups
 // g0 + 32 k (k < 4, g0 = 128 x warp + l): each store instruction writes 512
 // contiguous bytes (whole sectors), and the four groups' loads are in flight
-// together.  A relabelled id u is moved exactly when bit u of the moved
-// bitmap is set (perm[u] != u iff pinv[u] != u); a group with moved ids
-// gathers their working levels through pinv.
-__global__ void level_out_kernel(BfsDevState *st) {
+// together, as are the moved ids' maps and then their levels.  A relabelled id
+// u is moved exactly when bit u of the moved bitmap is set (perm[u] != u iff
+// pinv[u] != u); a group with moved ids gathers their working levels through
+// pinv.
+// The first block also copies the final state to the host (st->result, mapped
+// pinned memory), which saves the run a copy of its own.
+__global__ void __launch_bounds__(256, 4) level_out_kernel(BfsDevState *st) {
+  if (blockIdx.x == 0 && st->result != nullptr) {
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(st);
+    uint32_t *dst = reinterpret_cast<uint32_t *>(st->result);
+    for (uint32_t i = threadIdx.x; i < sizeof(BfsDevState) / 4; i += blockDim.x) dst[i] = src[i];
+  }
   int32_t *level = st->level;
   const uint8_t *lv8 = st->lv8;
   const uint32_t *moved = st->moved, *pinv = st->pinv;
@@ -149,18 +166,25 @@ __global__ void level_out_kernel(BfsDevState *st) {
         if (moved) mb[k] = (moved[u >> 5] >> (u & 31u)) & 0xFu;
       }
     }
+    // moved ids: the four groups' id maps together, then their levels
+    uint4 p[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (mb[k]) p[k] = __ldg(reinterpret_cast<const uint4 *>(pinv) + g0 + 32u * k);
+    uint32_t x[4][4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
-      const uint32_t g = g0 + 32u * k, u = g << 2;
-      if (g < n4) {
-        if (mb[k]) {
-          uint32_t x = 0;
+      const uint32_t id[4] = {p[k].x, p[k].y, p[k].z, p[k].w};
 #pragma unroll
-          for (uint32_t i = 0; i < 4; i++)
-            x |= (uint32_t)lv8[((mb[k] >> i) & 1u) ? pinv[u + i] : u + i] << (8u * i);
-          c[k] = x;
-        }
-        reinterpret_cast<int4 *>(level)[g] = output_levels4(c[k], level, u);
+      for (uint32_t i = 0; i < 4; i++)
+        x[k][i] = ((mb[k] >> i) & 1u) ? (uint32_t)lv8[id[i]] : (c[k] >> (8u * i)) & 0xFFu;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const uint32_t g = g0 + 32u * k;
+      if (g < n4) {
+        const uint32_t c4 = x[k][0] | (x[k][1] << 8) | (x[k][2] << 16) | (x[k][3] << 24);
+        reinterpret_cast<int4 *>(level)[g] = output_levels4(c4, level, g << 2);
       }
     }
   }
@@ -169,15 +193,6 @@ __global__ void level_out_kernel(BfsDevState *st) {
     const bool mv = moved && ((moved[u >> 5] >> (u & 31u)) & 1u);
     level[u] = output_level(lv8[mv ? pinv[u] : u], level, u);
   }
-}
-
-// The host template of the state, passed by value: seeding the state is a
-// kernel rather than a host-to-device copy, for the same reason.
-__global__ void seed_state_kernel(BfsDevState *st, BfsDevState s) {
-  static_assert(sizeof(BfsDevState) % 4 == 0, "state is copied in words");
-  const uint32_t *src = reinterpret_cast<const uint32_t *>(&s);
-  uint32_t *dst = reinterpret_cast<uint32_t *>(st);
-  for (uint32_t i = threadIdx.x; i < sizeof(BfsDevState) / 4; i += blockDim.x) dst[i] = src[i];
 }
 
 // Records, for the level being explored, which explore kernel ran.
@@ -193,59 +208,6 @@ struct BlockIndex {
   static constexpr int value = B == 128 ? 0 : B == 256 ? 1 : 2;
 };
 
-__device__ void init_state(BfsDevState *st, unsigned long long cond, int use_cond) {
-  const uint32_t r = st->root;                     // original id
-  const uint32_t ri = st->pinv ? st->pinv[r] : r;  // internal id
-  st->vis[ri >> 5] |= 1u << (ri & 31u);
-  st->prev[ri >> 5] |= 1u << (ri & 31u);
-  st->lv8[ri] = 0;
-  if (st->parent) st->parent[r] = (int32_t)r;
-  const bool expanded = ri < st->n_rows;  // run_bfs_cpu.hpp:31
-  uint32_t b = 0, e = 0;
-  if (expanded) {
-    b = st->indptr[ri];
-    e = st->indptr[ri + 1];
-  }
-  if (expanded && e > b) {
-    const uint32_t nch = edge_chunks(b, e - b, st->inds_off);
-    st->qb[0][0] = b;
-    st->qd[0][0] = e - b;
-    st->qc[0][0] = 0;
-    st->qc[0][1] = nch;
-    st->qv[0][0] = r;
-    st->F = 1;
-    st->EF = e - b;
-    st->EC = nch;
-  } else {
-    st->qc[0][0] = 0;
-    st->F = 0;
-    st->EF = 0;
-    st->EC = 0;
-  }
-  st->edges_count = expanded ? (unsigned long long)(e - b) : 0ull;
-  st->cur = 0;
-  st->lvl = 0;
-  st->reached = 1;
-  st->reached_prev = 1;
-  st->max_level = 0;
-  st->next_packed = 0;
-  st->next_edges = 0;
-  st->next_walk = 0;
-  st->skip_full = 0;
-  st->explore_done = 0;
-  st->done_blocks = 0;
-  st->lg_cursor = 0;
-  st->error = 0;
-  st->launches = 3;  // fill, init and the level output after the loop
-  st->arm = st->fixed_arm >= 0 ? st->fixed_arm : 0;
-  if (st->rec_cap > 0) {
-    st->rec_frontier[0] = st->F;
-    st->rec_edges[0] = st->EF;
-    st->rec_arm[0] = -1;
-  }
-  if (use_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond, st->F > 0);
-}
-
 // One warp: thread 0 seeds the root and the first frontier; with a fused
 // scheduler the warp then picks level 0's arm.
 __global__ void init_kernel(BfsDevState *st, unsigned long long cond, int use_cond) {
@@ -253,10 +215,12 @@ __global__ void init_kernel(BfsDevState *st, unsigned long long cond, int use_co
   if (blockIdx.x != 0 || threadIdx.x >= 32) return;
   const float *w = st->sched_w;
   if (w != nullptr) stage_weights(s_w, w);
-  if (threadIdx.x == 0) init_state(st, cond, use_cond);
+  if (threadIdx.x == 0) {
+    init_state(st, cond, use_cond);
+    st->launches += 1;
+  }
   __syncwarp();
-  if (w != nullptr && !narrow_next(st, st->F, st->EF))
-    fused_sched_pick(st, level_counters(st), s_w);
+  if (w != nullptr) fused_sched_pick(st, level_counters(st), s_w);
 }
 
 // ---- explore: LLB / SLB -----------------------------------------------------
@@ -1349,11 +1313,6 @@ cudaError_t launch_validate(const uint32_t *indptr, const uint32_t *inds, uint32
                                              parent_ok, bad);
   validate_vertices_kernel<<<1024, 256, 0, s>>>(n_cols, root, level, parent, witness,
                                                 parent_ok, bad);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_seed_state(BfsDevState *st, const BfsDevState &s, cudaStream_t stream) {
-  seed_state_kernel<<<1, 64, 0, stream>>>(st, s);
   return cudaGetLastError();
 }
 

@@ -20,7 +20,10 @@ inline uint32_t glb_chunk_edges(int ipt) { return 32u * (uint32_t)ipt * kGlbGrou
 
 // ---- narrow levels (narrow.cu) ----
 constexpr uint32_t kNarrowBlock = 512;
-constexpr uint32_t kNarrowHeavy = 128;       // degree of a heavy entry
+// Degree from which an entry goes to the list.  A warp takes a queue entry's
+// chunks 32 at a time, a chain of round trips each; R-MAT scale 12, whole BFS:
+// 57 us with 32 to 96, 63 with 128, 76 with 512, 105 with 1024.
+constexpr uint32_t kNarrowHeavy = 64;
 constexpr uint32_t kNarrowHeavyBound = 512;  // the same where only a bound on degrees is known
 // Largest level: 84 K edges (R-MAT scale 12) take 23 us in the two-kernel loop
 // and 14 on the cluster, 379 K (scale 14) take 86 us for the whole BFS there
@@ -42,7 +45,9 @@ BFS_HD bool narrow_level(uint32_t F, uint32_t EF, bool heavy) {
 BFS_HD bool narrow_next(const BfsDevState *st, uint32_t F, uint32_t EF) {
   return st->narrow != 0u && narrow_level(F, EF, EF - F + 1u > kNarrowHeavyBound);
 }
-// Arguments (BfsDevState*, conditional_handle, use_conditional); one cluster
+// Arguments (BfsDevState*, conditional_handle, use_conditional, int first);
+// first: seeds the root before it looks at the level (no init kernel then).
+// One cluster
 // of kNarrowBlock-thread blocks, grid = cluster size,
 // narrow_smem_bytes(parents) of dynamic shared memory.
 const void *narrow_kernel_fn(int cluster, bool parents);
@@ -53,7 +58,8 @@ cudaError_t narrow_cluster_size(int *cluster);
 
 // Kernel function pointers (for CUDA-graph kernel nodes and direct launches).
 // Every kernel takes (BfsDevState*) first; levelgen and init also take
-// (unsigned long long conditional_handle, int use_conditional).
+// (unsigned long long conditional_handle, int use_conditional), fill the
+// state's contents (BfsDevState).
 // parents: the variant that also records BFS-tree parents.
 const void *explore_kernel_fn(int arm, int ipt, bool parents);
 // The explore kernel that runs any arm: arguments (BfsDevState*, int arm),
@@ -67,14 +73,13 @@ const void *explore_any_kernel_fn(int ipt, bool parents);
 const void *levelgen_kernel_fn(bool parents);
 size_t levelgen_smem(bool parents);
 const void *init_kernel_fn();
-// fill clears the visited bitmaps (vis, prev: st->words words each), marks
+// fill writes the state, clears the visited bitmaps (vis, prev: st->words words each), marks
 // every working level unvisited and sets parents (when recorded) to -1.
 const void *fill_kernel_fn();
 // Writes the output levels (st->level, every entry) from the working levels;
-// runs once after the level loop.  Arguments (BfsDevState*).
+// runs once after the level loop; copies the state to its `result`, if any.
+// Arguments (BfsDevState*).
 const void *level_out_kernel_fn();
-// Writes the state st from a host copy with one small kernel.
-cudaError_t launch_seed_state(BfsDevState *st, const BfsDevState &s, cudaStream_t stream);
 
 cudaError_t launch_validate(const uint32_t *indptr, const uint32_t *inds, uint32_t n_rows,
                             uint32_t n_cols, uint32_t root, const int32_t *level,

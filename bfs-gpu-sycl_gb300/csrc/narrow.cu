@@ -47,6 +47,7 @@
 #include "device_util.cuh"
 #include "kernels.h"
 #include "bfs_sched_dev.cuh"
+#include "level_state.cuh"
 
 namespace bfsgb {
 namespace {
@@ -107,12 +108,11 @@ constexpr size_t narrow_smem(bool parents) {
 
 template <int C, bool PAR>
 __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kNarrowBlock, 1)
-    narrow_kernel(BfsDevState *__restrict__ st, unsigned long long cond, int use_cond) {
+    narrow_kernel(BfsDevState *__restrict__ st, unsigned long long cond, int use_cond, int first) {
   constexpr uint32_t NW = kNarrowBlock / 32;
   constexpr uint32_t kPer = kNarrowTile / kNarrowBlock;  // list entries per thread and tile
   static_assert(kPer * kNarrowBlock == kNarrowTile && NW <= 32, "block size");
   static_assert(kNarrowEntries <= 8u * kNarrowQueue, "the first level fits the queues");
-  static_assert(kSchedParams <= (int)kNarrowTile, "the model must fit a tile array");
   // positions are edge indexes counted from inds0, the 16-byte boundary at or
   // below inds
   extern __shared__ __align__(16) uint2 s_q[];  // [2][kNarrowQueue] (position, degree)
@@ -124,17 +124,29 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kNarrowBlock, 1)
   __shared__ uint32_t s_wsum[32];
   __shared__ NarrowCounters s_ctr[3];
   __shared__ NarrowCounters s_all;  // the cluster's totals
+  __shared__ float s_w[kSchedParams];  // rank 0: the scheduler's model
   __shared__ uint2 s_out;           // chunks of this block's part of the queue, at the end
 
   const uint32_t rank = cg::this_cluster().block_rank();
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t le_mask = (2u << lane) - 1u;
+  if (first) {
+    if (rank == 0 && tid == 0) init_state(st, cond, use_cond);
+    cg::this_cluster().sync();
+  }
+  const float *const w = st->sched_w;
   // F entries in all, L of them in this block's queue and G in the list
   uint32_t F = st->F, EF = st->EF, lvl = st->lvl, cur = st->cur;
   // no entry has more edges than this (every entry has at least one)
   const bool heavy = EF - F + 1u > kNarrowHeavyBound;
-  if (!narrow_level(F, EF, heavy)) {  // uniform over the cluster
+  const bool run = narrow_level(F, EF, heavy);  // uniform over the cluster
+  if (rank == 0 && w != nullptr && (run || first)) stage_weights(s_w, w);
+  if (!run) {
     if (rank == 0 && tid == 0) st->launches += 1;
+    if (first && F > 0u && w != nullptr && rank == 0) {
+      __syncthreads();
+      if (warp == 0) fused_sched_pick(st, level_counters(st), s_w);
+    }
     return;
   }
   uint32_t *const __restrict__ vis = st->vis;
@@ -448,9 +460,6 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(kNarrowBlock, 1)
     }
     if (rank == 0 && tid == 0) qc[F] = EC;
   }
-  const float *w = st->sched_w;
-  float *s_w = reinterpret_cast<float *>(s_beg);
-  if (rank == 0 && F > 0u && w != nullptr) stage_weights(s_w, w);
   if (rank == 0 && tid == 0) {
     st->F = F;
     st->EF = EF;

@@ -58,9 +58,8 @@ constexpr uint32_t kMaxV = BFS_NOALLOC_MAX_VERTICES;
 constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 // layout of the scratch array
 constexpr size_t kStateOff = 0;
-constexpr size_t kBadOff = align256(sizeof(BfsDevState));
 constexpr size_t kWordsMax = (((size_t)kMaxV + 31) / 32 + 31) / 32 * 32;
-constexpr size_t kVisOff = kBadOff + 256;
+constexpr size_t kVisOff = align256(sizeof(BfsDevState));
 constexpr size_t kPrevOff = kVisOff + align256(kWordsMax * 4);
 constexpr size_t kQ4 = align256((size_t)kMaxV * 4);
 constexpr size_t kQp4 = align256(((size_t)kMaxV + 1) * 4);
@@ -78,16 +77,6 @@ int g_narrow[kMaxDevices] = {};   // narrow-level cluster size (0: not run)
 
 constexpr int kArm = 4;  // GLB, 256 threads
 constexpr int kIpt = 4;
-
-// Writes the loop state from its by-value argument and clears the error
-// counter (no host-to-device copy of a host buffer is needed).
-__global__ void noalloc_state_kernel(BfsDevState s, BfsDevState *dst,
-                                     unsigned long long *bad) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    *dst = s;
-    *bad = 0ull;
-  }
-}
 
 bfs_status setup_device(int dev) {
   std::lock_guard<std::mutex> lk(g_setup_mutex);
@@ -177,31 +166,28 @@ extern "C" bfs_status bfs_run_device_noalloc(const uint32_t *d_indptr, const uin
   h.level_cap = n_cols + 1u;
   h.rec_cap = 0;  // no per-level record in this entry point
   BfsDevState *st = (BfsDevState *)(base + kStateOff);
-  unsigned long long *bad = (unsigned long long *)(base + kBadOff);
 
-  // State, CSC check, fill, init and the first narrow levels are queued
+  // State, fill, CSC check, init and the first narrow levels are queued
   // without a read-back: a malformed CSC leaves the state without rows, so
   // that init queues no root and no later kernel follows an edge.
   const int cluster = g_narrow[dev];
   h.narrow = cluster > 0 ? 1u : 0u;
-  noalloc_state_kernel<<<1, 32, 0, s>>>(h, st, bad);
-  NK(cudaGetLastError());
-  NK(launch_check_csc(d_indptr, d_inds, n_cols, nnz, bad, s, &st->n_rows));
-  unsigned long long no_cond = 0;
-  int zero = 0;
-  void *fill_args[] = {&st};
+  void *fill_args[] = {&st, &h};
   NK(cudaLaunchKernel(fill_kernel_fn(), dim3(g_grid[dev][1]), dim3(256), fill_args, 0, s));
-  void *lg_args[] = {&st, &no_cond, &zero};
-  NK(cudaLaunchKernel(init_kernel_fn(), dim3(1), dim3(32), lg_args, 0, s));
-  unsigned long long h_bad = 0;
-  NK(cudaMemcpyAsync(&h_bad, bad, sizeof(h_bad), cudaMemcpyDeviceToHost, s));
+  NK(launch_check_csc(d_indptr, d_inds, n_cols, nnz, &st->bad, s, &st->n_rows));
+  unsigned long long no_cond = 0;
+  int zero = 0, first = 1;
+  void *lg_args[] = {&st, &no_cond, &zero, &first};
+  if (cluster == 0)
+    NK(cudaLaunchKernel(init_kernel_fn(), dim3(1), dim3(32), lg_args, 0, s));
   for (;;) {
     if (cluster > 0)
       NK(cudaLaunchKernel(narrow_kernel_fn(cluster, false), dim3(cluster), dim3(kNarrowBlock),
                           lg_args, narrow_smem_bytes(false), s));
     NK(cudaMemcpyAsync(&h, st, sizeof(h), cudaMemcpyDeviceToHost, s));
     NK(cudaStreamSynchronize(s));
-    if (h_bad) return fail(BFS_ERR_GRAPH, "malformed CSC: " + std::to_string(h_bad) + " errors");
+    first = 0;
+    if (h.bad) return fail(BFS_ERR_GRAPH, "malformed CSC: " + std::to_string(h.bad) + " errors");
     if (h.F == 0) break;
     void *ex_args[] = {&st};
     NK(cudaLaunchKernel(explore_kernel_fn(kArm, kIpt, false), dim3(g_grid[dev][0]), dim3(arm_block(kArm)),
@@ -209,7 +195,8 @@ extern "C" bfs_status bfs_run_device_noalloc(const uint32_t *d_indptr, const uin
     NK(cudaLaunchKernel(levelgen_kernel_fn(false), dim3(g_grid[dev][1]), dim3(kLevelgenBlock),
                         lg_args, levelgen_smem(false), s));
   }
-  NK(cudaLaunchKernel(level_out_kernel_fn(), dim3(g_grid[dev][1]), dim3(256), fill_args, 0, s));
+  void *ex_out[] = {&st};
+  NK(cudaLaunchKernel(level_out_kernel_fn(), dim3(g_grid[dev][1]), dim3(256), ex_out, 0, s));
   NK(cudaStreamSynchronize(s));
   const uint32_t err = h.error;
   if (err & BFS_DEVERR_LEVEL_LIMIT)
