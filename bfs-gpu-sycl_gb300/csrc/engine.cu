@@ -60,7 +60,15 @@ size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // ---- handle lifetime ---------------------------------------------------------
 
+static void free_queued_run(QueuedRun &q) {
+  if (q.result) cudaFreeHost(q.result);
+  if (q.e0) cudaEventDestroy(q.e0);
+  if (q.e1) cudaEventDestroy(q.e1);
+}
+
 static void free_workspace(bfs_graph *g) {
+  for (auto &q : g->ahead) free_queued_run(q);
+  g->ahead.clear();
   for (auto &kv : g->graphs) {
     if (kv.second.exec) cudaGraphExecDestroy(kv.second.exec);
     if (kv.second.graph) cudaGraphDestroy(kv.second.graph);
@@ -564,9 +572,32 @@ bfs_status ensure_hub(bfs_graph *g) {
   return rc;
 }
 
+// Errors and statistics of a finished run with final state r.
+static bfs_status collect_run(const BfsDevState &r, cudaEvent_t e0, cudaEvent_t e1,
+                              uint32_t launches, bfs_stats *stats) {
+  if (r.error & BFS_DEVERR_LEVEL_LIMIT)
+    return fail(BFS_ERR_LEVEL_LIMIT, "level loop exceeded n_cols + 1 levels");
+  if (r.error) return fail(BFS_ERR_DEVICE, "device error flag " + std::to_string(r.error));
+  if (!stats) return BFS_OK;
+  float ms = 0.f;
+  CK(cudaEventElapsedTime(&ms, e0, e1));
+  stats->edges_count = r.edges_count;
+  stats->reached = r.reached;
+  stats->num_levels = r.max_level + 1;
+  stats->device_ms = ms;
+  stats->launches = launches;
+  stats->recorded = 0;
+  return BFS_OK;
+}
+
+static void clear_level_times(bfs_stats *stats) {
+  std::memset(stats->level_explore_ms, 0, sizeof(stats->level_explore_ms));
+  std::memset(stats->level_gen_ms, 0, sizeof(stats->level_gen_ms));
+}
+
 bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts_in,
                            int32_t *levels_dev, int32_t *parents_dev, bfs_stats *stats,
-                           LevelTimer *timer, const std::function<bfs_status()> *after_launch) {
+                           LevelTimer *timer, QueuedRun *queued) {
   if (!g || !levels_dev) return fail(BFS_ERR_INVALID_ARG, "null graph or level buffer");
   if (root >= g->n_cols) return fail(BFS_ERR_ROOT, "root out of range");
   bfs_options o;
@@ -601,8 +632,7 @@ bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts_
   if (o.record >= 2 && stats) {
     g->prof_explore = stats->level_explore_ms;
     g->prof_gen = stats->level_gen_ms;
-    std::memset(stats->level_explore_ms, 0, sizeof(stats->level_explore_ms));
-    std::memset(stats->level_gen_ms, 0, sizeof(stats->level_gen_ms));
+    clear_level_times(stats);
   }
   bfs_status hrc = ensure_hub(g);
   if (hrc != BFS_OK) return hrc;
@@ -654,8 +684,14 @@ bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts_
       s.sched_avg_deg_x = gc.avg_deg_x;
     }
   }
-  CK(cudaEventRecord(g->ev0, g->stream));
-  s.result = graph_loop ? g->h_st : nullptr;  // written by the output pass
+  QueuedRun own;
+  own.result = g->h_st;
+  own.e0 = g->ev0;
+  own.e1 = g->ev1;
+  const bool ahead = queued != nullptr && graph_loop && o.record == 0;
+  const QueuedRun &q = ahead ? *queued : own;
+  CK(cudaEventRecord(q.e0, g->stream));
+  s.result = graph_loop ? q.result : nullptr;  // written by the output pass
   void *fill_args[] = {&g->d_st, &s};
   CK(cudaLaunchKernel(fill_kernel_fn(), dim3(g->num_sms * 4), dim3(256), fill_args, 0, g->stream));
   uint32_t launches = 0;
@@ -666,14 +702,10 @@ bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts_
     if (rc != BFS_OK) return rc;
     launches = g->host_launches;
   }
-  CK(cudaEventRecord(g->ev1, g->stream));
-  if (after_launch) {
-    rc = (*after_launch)();
-    if (rc != BFS_OK) {
-      cudaStreamSynchronize(g->stream);
-      return rc;
-    }
-  }
+  CK(cudaEventRecord(q.e1, g->stream));
+  if (stats && o.record < 2) clear_level_times(stats);
+  if (queued) queued->pending = ahead;
+  if (ahead) return BFS_OK;
   if (graph_loop) {
     CK(cudaStreamSynchronize(g->stream));
   } else {
@@ -681,22 +713,9 @@ bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts_
     if (rc != BFS_OK) return rc;
   }
   const BfsDevState &r = *g->h_st;
-  if (r.error & BFS_DEVERR_LEVEL_LIMIT)
-    return fail(BFS_ERR_LEVEL_LIMIT, "level loop exceeded n_cols + 1 levels");
-  if (r.error) return fail(BFS_ERR_DEVICE, "device error flag " + std::to_string(r.error));
+  rc = collect_run(r, q.e0, q.e1, launches ? launches : r.launches, stats);
+  if (rc != BFS_OK) return rc;
   if (stats) {
-    float ms = 0.f;
-    CK(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
-    stats->edges_count = r.edges_count;
-    stats->reached = r.reached;
-    stats->num_levels = r.max_level + 1;
-    stats->device_ms = ms;
-    stats->launches = launches ? launches : r.launches;
-    stats->recorded = 0;
-    if (o.record < 2) {
-      std::memset(stats->level_explore_ms, 0, sizeof(stats->level_explore_ms));
-      std::memset(stats->level_gen_ms, 0, sizeof(stats->level_gen_ms));
-    }
     if (o.record) {
       const uint32_t nrec = std::min<uint32_t>(r.lvl + 1, BFS_MAX_RECORDED_LEVELS);
       stats->recorded = nrec;
@@ -856,21 +875,31 @@ bfs_status bfs_run(bfs_graph *g, uint32_t root, const bfs_options *opts, int32_t
   const size_t bytes = sizeof(int32_t) * (size_t)g->n_cols;
   if (!g->d_out_levels) CK(dev_malloc(&g->d_out_levels, bytes));
   if (parents_host && !g->d_out_parents) CK(dev_malloc(&g->d_out_parents, bytes));
+  // the copies follow the run on its stream, without a wait in between
+  QueuedRun q;
+  q.result = g->h_st;
+  q.e0 = g->ev0;
+  q.e1 = g->ev1;
   bfs_status rc = run_device_impl(g, root, opts, g->d_out_levels,
-                                  parents_host ? g->d_out_parents : nullptr, stats, nullptr);
+                                  parents_host ? g->d_out_parents : nullptr, stats, nullptr, &q);
   if (rc != BFS_OK) return rc;
   CK(cudaMemcpyAsync(levels_host, g->d_out_levels, bytes, cudaMemcpyDeviceToHost, g->stream));
   if (parents_host)
     CK(cudaMemcpyAsync(parents_host, g->d_out_parents, bytes, cudaMemcpyDeviceToHost, g->stream));
   CK(cudaStreamSynchronize(g->stream));
-  return BFS_OK;
+  return q.pending ? collect_run(*q.result, q.e0, q.e1, q.result->launches, stats) : BFS_OK;
 }
 
 // Runs i and i + 1 write device buffers of alternating slots; run i's copy
 // to the host is queued on the copy stream once run i + 1 is queued, so it
 // overlaps run i + 1, and run i + 2 waits on the main stream for that copy
-// before it overwrites the slot.  Device-to-host copies into pageable memory
-// return only when done, so with pageable buffers the runs are serial.
+// before it overwrites the slot.  Up to kRunsAhead runs are queued before the
+// host waits for the first (waiting for each run's state before the next was
+// queued left the GPU idle for about 50 us per root).  Device-to-host copies
+// into pageable memory return only when done, so with pageable buffers the
+// runs are serial.
+constexpr uint32_t kRunsAhead = 32;
+
 static bfs_status run_roots_impl(bfs_graph *g, const uint32_t *roots, uint32_t n_roots,
                                  const bfs_options *opts, int32_t *const *levels_host,
                                  int32_t *const *parents_host, bfs_stats *stats) {
@@ -883,7 +912,19 @@ static bfs_status run_roots_impl(bfs_graph *g, const uint32_t *roots, uint32_t n
   if (!g->ev_ready) CK(cudaEventCreateWithFlags(&g->ev_ready, cudaEventDisableTiming));
   for (auto &e : g->ev_copied)
     if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  // queues the copy of finished run j (its device buffers are slot j & 1)
+  while (g->ahead.size() < std::min(n_roots, kRunsAhead)) {
+    g->ahead.emplace_back();
+    QueuedRun &q = g->ahead.back();
+    cudaError_t e = cudaMallocHost(&q.result, sizeof(BfsDevState));
+    if (e == cudaSuccess) e = cudaEventCreate(&q.e0);
+    if (e == cudaSuccess) e = cudaEventCreate(&q.e1);
+    if (e != cudaSuccess) {
+      free_queued_run(q);
+      g->ahead.pop_back();
+      CK(e);
+    }
+  }
+  // queues the copy of run j (its device buffers are slot j & 1)
   auto copy_out = [&](uint32_t j) -> bfs_status {
     const int slot = (int)(j & 1u);
     CK(cudaStreamWaitEvent(g->copy_stream, g->ev_ready, 0));
@@ -895,19 +936,30 @@ static bfs_status run_roots_impl(bfs_graph *g, const uint32_t *roots, uint32_t n
     CK(cudaEventRecord(g->ev_copied[slot], g->copy_stream));
     return BFS_OK;
   };
-  for (uint32_t i = 0; i < n_roots; i++) {
-    const int slot = (int)(i & 1u);
-    if (i >= 2) CK(cudaStreamWaitEvent(g->stream, g->ev_copied[slot], 0));
-    // run i-1's copy is issued after run i is queued, so that it does not
-    // hold up the start of run i, and before the wait for run i
-    const std::function<bfs_status()> prev_copy = [&]() { return copy_out(i - 1); };
-    // returns after the run has finished (it reads the device state back)
-    bfs_status rc = run_device_impl(g, roots[i], opts, g->d_ring[slot][0],
-                                    parents_host ? g->d_ring[slot][1] : nullptr,
-                                    stats ? stats + i : nullptr, nullptr,
-                                    i > 0 ? &prev_copy : nullptr);
-    if (rc != BFS_OK) return rc;
-    CK(cudaEventRecord(g->ev_ready, g->stream));  // run i has finished
+  for (uint32_t w0 = 0; w0 < n_roots; w0 += kRunsAhead) {
+    const uint32_t w1 = std::min(n_roots, w0 + kRunsAhead);
+    for (uint32_t i = w0; i < w1; i++) {
+      const int slot = (int)(i & 1u);
+      if (i >= 2) CK(cudaStreamWaitEvent(g->stream, g->ev_copied[slot], 0));
+      bfs_status rc = run_device_impl(g, roots[i], opts, g->d_ring[slot][0],
+                                      parents_host ? g->d_ring[slot][1] : nullptr,
+                                      stats ? stats + i : nullptr, nullptr, &g->ahead[i - w0]);
+      if (rc != BFS_OK) return rc;
+      // run i - 1's copy is issued after run i is queued, so that it does not
+      // hold up the start of run i, and before run i's end is recorded
+      if (i > 0) {
+        rc = copy_out(i - 1);
+        if (rc != BFS_OK) return rc;
+      }
+      CK(cudaEventRecord(g->ev_ready, g->stream));  // run i has finished
+    }
+    CK(cudaStreamSynchronize(g->stream));
+    for (uint32_t i = w0; i < w1; i++) {
+      const QueuedRun &q = g->ahead[i - w0];
+      if (!q.pending) continue;
+      bfs_status rc = collect_run(*q.result, q.e0, q.e1, q.result->launches, stats ? stats + i : nullptr);
+      if (rc != BFS_OK) return rc;
+    }
   }
   return copy_out(n_roots - 1);
 }
@@ -925,7 +977,9 @@ bfs_status bfs_run_roots(bfs_graph *g, const uint32_t *roots, uint32_t n_roots,
   if (n_roots == 0) return BFS_OK;
   CK(cudaSetDevice(g->device));
   const bfs_status rc = run_roots_impl(g, roots, n_roots, opts, levels_host, parents_host, stats);
-  // no copy into the caller's buffers is left in flight, also after an error
+  // no run and no copy into the caller's buffers is left in flight, also after
+  // an error
+  if (rc != BFS_OK) cudaStreamSynchronize(g->stream);
   if (g->copy_stream) {
     const cudaError_t e = cudaStreamSynchronize(g->copy_stream);
     if (rc == BFS_OK && e != cudaSuccess) return fail(BFS_ERR_CUDA, cudaGetErrorString(e));

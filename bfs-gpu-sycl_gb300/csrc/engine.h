@@ -2,7 +2,6 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include <functional>
 #include <map>
 #include <vector>
 
@@ -28,13 +27,20 @@ struct LevelTimer {
   void (*after)(void *ctx, bfs_graph *g, uint32_t level, int arm) = nullptr;
 };
 
-// after_launch (optional) runs once the BFS is queued on the handle's stream
-// and before the call waits for it: work issued there (e.g. copies on another
-// stream) is queued ahead of the run's final state read.
+// A run that is queued without waiting for it: where its final state goes
+// (pinned), the events around it, and whether it still has to be collected
+// (plans that the host drives are finished when run_device_impl returns).
+struct QueuedRun {
+  BfsDevState *result = nullptr;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  bool pending = false;
+};
+
+// With `queued`, a CUDA-graph run without a record is queued on the handle's
+// stream and left to collect_run once the stream has been waited for.
 bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts,
                            int32_t *levels_dev, int32_t *parents_dev, bfs_stats *stats,
-                           LevelTimer *timer,
-                           const std::function<bfs_status()> *after_launch = nullptr);
+                           LevelTimer *timer, QueuedRun *queued = nullptr);
 // Launches one explore kernel on the handle's stream for a frontier of F
 // entries and EF edges; persistent = full persistent grid (as in the graph
 // loop) instead of a grid sized to the frontier.
@@ -76,6 +82,7 @@ struct bfs_graph {
   cudaStream_t stream = nullptr;
   cudaStream_t copy_stream = nullptr;  // bfs_run_roots: device-to-host copies
   cudaEvent_t ev_ready = nullptr, ev_copied[2] = {nullptr, nullptr};
+  std::vector<bfsgb::QueuedRun> ahead;  // bfs_run_roots: runs queued at a time
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t lvl_ev[3] = {nullptr, nullptr, nullptr};  // per-level kernel timing
   float *prof_explore = nullptr;  // host arrays filled by the host loop (record == 2)
