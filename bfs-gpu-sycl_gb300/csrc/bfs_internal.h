@@ -103,6 +103,7 @@ struct BfsDevState {
   uint32_t n_rows, n_cols;
   uint32_t words;        // bitmap words (padded)
   uint32_t root;
+  uint32_t root_id;      // the root's internal id (written by init)
   // workspace
   uint32_t *vis;
   uint32_t *prev;

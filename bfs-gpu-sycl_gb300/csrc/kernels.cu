@@ -427,11 +427,17 @@ __global__ void __launch_bounds__(B, (MinBlocks<B, U, STRIDED>::value))
 // the 64 registers of a 1024-thread block (4 chunks per group spill).  One
 // chunk does better where a warp has few groups to walk or entries of few
 // chunks: R-MAT scale 19 173 us (GLB) instead of 199 with two, scale 21 253
-// instead of 272, ER 3 M vertices 413 instead of 430; scale 23 615 either way;
-// scale 25 2.00 ms instead of 1.92.  So levels from kGroupChunks on walk two.
-constexpr uint32_t kGroupChunks = 1u << 25;
+// instead of 272, ER 3 M vertices 413 instead of 430; scale 23 with edge factor
+// 8 (levels of 23 M and 13 M chunks) 619 us instead of 609; scale 25 2.00 ms
+// instead of 1.92.  So levels from kGroupChunks on walk two.
+constexpr uint32_t kGroupChunks = 1u << 24;
+// Packed claims (below) pay from about here on: without them scale 23 with
+// edge factor 8 and rows < cols 592 us instead of 617, scale 22 with rows <
+// cols 505 instead of 517; with them scale 24 with rows < cols 1592 instead of
+// 1650, scale 25 1.96 ms instead of 2.09, scale 23 616 us instead of 645.
+constexpr uint32_t kPackedChunks = 1u << 25;
 
-template <int U, bool PAR, bool HUB>
+template <int U, bool PAR, bool HUB, bool PACKED>
 __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict__ st,
                                                    uint32_t F, uint32_t gw,
                                                    uint32_t total_warps, uint32_t *s_hub,
@@ -453,17 +459,19 @@ __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict
   const uint32_t hi4 = (st->nnz + off) >> 2;
   uint32_t *vis = st->vis;
   const uint32_t *vis_c = vis;  // plain loads of the visited words
+  // stands in for the slots outside an entry's edges: no mask goes with a chunk
+  const uint32_t visited = st->root_id;
   const uint32_t s_hub_addr = HUB ? (uint32_t)__cvta_generic_to_shared(s_hub) : 0u;
   int32_t *parent = PAR ? st->parent : nullptr;
   const uint32_t *perm = PAR ? st->perm : nullptr;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t le_mask = (2u << lane) - 1u;  // lanes 0 .. lane (all for lane 31)
   const uint64_t pol = evict_first_policy();
-  // Claims wait in the warp's 32 slots of s_claim (target, queue entry) and
-  // are made 32 at a time, with the parents' chain of loads and the store
-  // side by side.  Made slot by slot, with a few lanes each, they took R-MAT
-  // scale 25 with parents from 4.0 to 8.4 ms per BFS (scale 23 0.91 to 1.70,
-  // scale 21 0.33 to 0.50), and without parents from 1.96 to 2.09.
+  // PACKED: claims wait in the warp's 32 slots of s_claim (target, queue entry)
+  // and are made 32 at a time, with the parents' chain of loads and the store
+  // side by side; otherwise a lane makes its own, slot by slot.  With parents
+  // packing takes R-MAT scale 25 from 8.4 to 4.0 ms per BFS (scale 23 1.70 to
+  // 0.91, scale 21 0.50 to 0.33).
   uint32_t waiting = 0;
   auto flush_claims = [&]() {
     __syncwarp();
@@ -506,13 +514,24 @@ __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict
     load_window();
     uint32_t wlast = __shfl_sync(kFull, bnd, 31);
     // Resolves the U rounds of chunks starting at chunk `base` and issues
-    // their 16-byte loads: q (slots), m (valid-slot mask, bit i = slot i),
-    // fr (source id, with parents).
-    auto resolve = [&](uint32_t base, uint4 (&q)[U], uint32_t (&m)[U], uint32_t (&fr)[U]) {
+    // their 16-byte loads: q (slots; `visited` outside the entry's edges), fr
+    // (queue entry, with parents).
+    // chunks [f0, f1) of the range hold four edges of entry cur each
+    uint32_t f0 = ((cb + 3u) >> 2) - cd, f1 = min((ce >> 2) - cd, w1);
+    auto resolve = [&](uint32_t base, uint4 (&q)[U], uint32_t (&fr)[U]) {
 #pragma unroll
       for (int u = 0; u < U; u++) {
         const uint32_t rb = base + 32u * u;
         const uint32_t x = rb + lane;
+        // warp-uniform: a round inside one entry, most rounds of the entries of
+        // hundreds of edges that make up the largest levels (with the slot masks
+        // gone from the probes, R-MAT scale 25 1938 -> 1903 us, scale 23 643 ->
+        // 631, scale 21 270 -> 266)
+        if (rb >= f0 && rb + 32u <= f1) {
+          q[u] = ld_stream4(inds4 + (x + cd), pol);
+          fr[u] = PAR ? cur : 0u;
+          continue;
+        }
         if (wlast < rb || wlast - rb < 31u) {  // warp-uniform
           c0 = cur;
           load_window();
@@ -527,21 +546,23 @@ __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict
         const uint32_t se = __shfl_sync(kFull, we, srcl);
         const uint32_t d = k ? sd : cd, b = k ? sb : cb, e = k ? se : ce;
         fr[u] = PAR ? cur + k : 0u;
-        m[u] = 0u;
-        q[u] = make_uint4(0u, 0u, 0u, 0u);
+        q[u] = make_uint4(visited, visited, visited, visited);
         if (x < w1) {
           const uint32_t a4 = x + d;    // chunk index from inds0
           const uint32_t p0 = a4 << 2;  // position of its slot 0
           const uint32_t lo = b > p0 ? b - p0 : 0u;        // 0 .. 3
           const uint32_t hi = e - p0 < 4u ? e - p0 : 4u;   // 1 .. 4
-          m[u] = (0xFu >> (4u - hi)) & (0xFu << lo);
           if (a4 >= lo4 && a4 < hi4) {
             q[u] = ld_stream4(inds4 + a4, pol);
+            if (lo > 0u) q[u].x = visited;
+            if (lo > 1u || hi < 2u) q[u].y = visited;
+            if (lo > 2u || hi < 3u) q[u].z = visited;
+            if (hi < 4u) q[u].w = visited;
           } else {  // a chunk that reaches outside inds: its valid slots only
-            uint32_t t[4] = {0u, 0u, 0u, 0u};
+            uint32_t t[4];
 #pragma unroll
-            for (int i = 0; i < 4; i++)
-              if ((m[u] >> i) & 1u) t[i] = ld_stream(inds0 + p0 + i, pol);
+            for (uint32_t i = 0; i < 4; i++)
+              t[i] = i >= lo && i < hi ? ld_stream(inds0 + p0 + i, pol) : visited;
             q[u] = make_uint4(t[0], t[1], t[2], t[3]);
           }
         }
@@ -553,16 +574,18 @@ __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict
           cd = __shfl_sync(kFull, wd, sl);
           cb = __shfl_sync(kFull, wb, sl);
           ce = __shfl_sync(kFull, we, sl);
+          f0 = ((cb + 3u) >> 2) - cd;
+          f1 = min((ce >> 2) - cd, w1);
         }
       }
     };
     // Probes of the U chunks of a lane, branch-free: for every slot a
     // predicated shared load of the hub word (hub ids only), then a
-    // predicated global load of the visited word (valid slots the hub word
-    // did not show visited); a slot whose word shows its bit clear gets a
+    // predicated global load of the visited word (slots the hub word did not
+    // show visited); a slot whose word shows its bit clear gets a
     // bit in need[u].  Only then, behind one branch per chunk, the claims,
     // packed into the warp's waiting slots.
-    auto probe = [&](const uint4 (&q)[U], const uint32_t (&m)[U], const uint32_t (&fr)[U]) {
+    auto probe = [&](const uint4 (&q)[U], const uint32_t (&fr)[U]) {
       uint32_t need[U];
 #pragma unroll
       for (int u = 0; u < U; u++) {
@@ -572,51 +595,65 @@ __device__ __forceinline__ void explore_chunk_body(const BfsDevState *__restrict
         for (int i = 0; i < 4; i++) {
           const uint32_t n = n4[i];
           const uint32_t bit = 1u << (n & 31u);
-          uint32_t act = (m[u] >> i) & 1u;
+          uint32_t word;
           if (HUB) {
-            uint32_t h = 0u;
-            ld_shared_if(h, s_hub_addr + ((n >> 5) << 2), act & (n < hub_lim ? 1u : 0u));
-            act &= (h & bit) ? 0u : 1u;
+            word = 0u;
+            ld_shared_if(word, s_hub_addr + ((n >> 5) << 2), n < hub_lim ? 1u : 0u);
+            ld_global_if(word, vis_c + (n >> 5), (word & bit) ? 0u : 1u);
+          } else {  // the slots outside an entry make no request
+            word = kFull;
+            ld_global_if(word, vis_c + (n >> 5), n != visited ? 1u : 0u);
           }
-          uint32_t word = bit;  // "visited" unless loaded
-          ld_global_if(word, vis_c + (n >> 5), act);
           need[u] |= ((word & bit) ? 0u : 1u) << i;
         }
       }
+      if constexpr (PACKED) {
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        if (!__any_sync(kFull, need[u] != 0u)) continue;
-        const uint32_t n4[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
+        for (int u = 0; u < U; u++) {
+          if (!__any_sync(kFull, need[u] != 0u)) continue;
+          const uint32_t n4[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const uint32_t bal = __ballot_sync(kFull, (need[u] >> i) & 1u);
-          const uint32_t num = __popc(bal);
-          if (waiting + num > 32u) flush_claims();  // uniform
-          if ((need[u] >> i) & 1u)
-            s_claim[waiting + __popc(bal & (le_mask >> 1))] = make_uint2(n4[i], fr[u]);
-          waiting += num;
+          for (int i = 0; i < 4; i++) {
+            const uint32_t bal = __ballot_sync(kFull, (need[u] >> i) & 1u);
+            const uint32_t num = __popc(bal);
+            if (waiting + num > 32u) flush_claims();  // uniform
+            if ((need[u] >> i) & 1u)
+              s_claim[waiting + __popc(bal & (le_mask >> 1))] = make_uint2(n4[i], fr[u]);
+            waiting += num;
+          }
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+          if (need[u] == 0u) continue;
+          const uint32_t n4[4] = {q[u].x, q[u].y, q[u].z, q[u].w};
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            if (!((need[u] >> i) & 1u)) continue;
+            red_or(vis + (n4[i] >> 5), 1u << (n4[i] & 31u));
+            if (HUB && n4[i] < hub_lim) atomicOr(s_hub + (n4[i] >> 5), 1u << (n4[i] & 31u));
+          }
         }
       }
     };
     // Software pipeline: the loads of the next U rounds are issued before
     // the probes of the current ones, so that they overlap.
     uint4 q[U], q2[U];
-    uint32_t m[U], m2[U], fr[U], fr2[U];
-    resolve(w0, q, m, fr);
+    uint32_t fr[U], fr2[U];
+    resolve(w0, q, fr);
     for (uint32_t base = w0; base < w1; base += kRound) {
       const bool more = base + kRound < w1;  // warp-uniform; no overflow: w1 < 2^32 - kRound
-      if (more) resolve(base + kRound, q2, m2, fr2);
-      probe(q, m, fr);
+      if (more) resolve(base + kRound, q2, fr2);
+      probe(q, fr);
       if (!more) break;
 #pragma unroll
       for (int u = 0; u < U; u++) {
         q[u] = q2[u];
-        m[u] = m2[u];
         fr[u] = fr2[u];
       }
     }
   }
-  flush_claims();
+  if constexpr (PACKED) flush_claims();
 }
 
 // The GLB arms' own kernel (the engine runs GLB levels in explore_any; the
@@ -628,9 +665,9 @@ __global__ void __launch_bounds__(B, 1024 / B)
   if (F == 0) return;
   note_arm<1 * 3 + BlockIndex<B>::value>(st);
   __shared__ uint2 s_claim[B];
-  explore_chunk_body<1, PAR, false>(st, F, blockIdx.x * (B / 32) + (threadIdx.x >> 5),
-                                    gridDim.x * (B / 32), nullptr, 0u,
-                                    s_claim + (threadIdx.x & ~31u));
+  explore_chunk_body<1, PAR, false, PAR>(st, F, blockIdx.x * (B / 32) + (threadIdx.x >> 5),
+                                         gridDim.x * (B / 32), nullptr, 0u,
+                                         s_claim + (threadIdx.x & ~31u));
 }
 
 // Whole grid, after a level's claims: the last block to finish looks which
@@ -715,10 +752,18 @@ __global__ void __launch_bounds__(kAnyBlock, 1)
     }
     const uint32_t gw = blockIdx.x * (kAnyBlock / 32) + (t >> 5);
     const uint32_t gws = gridDim.x * (kAnyBlock / 32), lim = use ? hw * 32u : 0u;
-    if (st->EC >= kGroupChunks)
-      explore_chunk_body<2, PAR, true>(st, F, gw, gws, s_hub, lim, s_claim + (t & ~31u));
+    uint2 *const claims = s_claim + (t & ~31u);
+    const uint32_t EC = st->EC;
+    // the body without the filter has no probe for the slots outside an entry;
+    // with parents, and on wide levels, a second body costs more in spills
+    if (EC >= kPackedChunks || (PAR && EC >= kGroupChunks))
+      explore_chunk_body<2, PAR, true, true>(st, F, gw, gws, s_hub, lim, claims);
+    else if (EC >= kGroupChunks)
+      explore_chunk_body<2, PAR, true, PAR>(st, F, gw, gws, s_hub, lim, claims);
+    else if (use || PAR)
+      explore_chunk_body<1, PAR, true, PAR>(st, F, gw, gws, s_hub, lim, claims);
     else
-      explore_chunk_body<1, PAR, true>(st, F, gw, gws, s_hub, lim, s_claim + (t & ~31u));
+      explore_chunk_body<1, PAR, false, PAR>(st, F, gw, gws, nullptr, 0u, claims);
     if (full < st->skip_classes && st->EF >= st->skip_min_edges) find_full_classes(st, full);
   } else if (bi == 2) {
     const uint32_t v = t >> 9, o = v * 513u;

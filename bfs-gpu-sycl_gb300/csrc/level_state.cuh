@@ -11,6 +11,7 @@ namespace bfsgb {
 __device__ __forceinline__ void init_state(BfsDevState *st, unsigned long long cond, int use_cond) {
   const uint32_t r = st->root;                     // original id
   const uint32_t ri = st->pinv ? st->pinv[r] : r;  // internal id
+  st->root_id = ri;
   st->vis[ri >> 5] |= 1u << (ri & 31u);
   st->prev[ri >> 5] |= 1u << (ri & 31u);
   st->lv8[ri] = 0;
