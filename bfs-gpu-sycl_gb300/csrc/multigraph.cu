@@ -37,6 +37,7 @@
 
 namespace bfsgb {
 
+constexpr uint32_t kShareEdges = 1u << 17;
 constexpr uint32_t kMultiMaxVertices = 1u << 18;  // 32 KiB shared bitmap
 
 struct MultiDesc {
@@ -79,9 +80,10 @@ struct MultiTile {
 // One level of one graph over tiles tile0, tile0 + tstride, ... of B
 // frontier entries (LLB form): block exclusive scan over the tile, entries
 // without edges dropped, the tile's edges split evenly over the warps, owners
-// resolved per warp round.  With IPT = 4 a round deals 16-byte chunks of the
-// edge array, one per lane -- four edges in flight for one owner resolution;
-// otherwise IPT rounds of single edges.  A claim is an atomicOr on the visited
+// resolved per warp round.  With IPT of 2 or more a round deals 16-byte chunks
+// of the edge array, one per lane -- four edges in flight for one owner
+// resolution (two rounds of single edges at IPT = 2 took 100 us instead of 74 on
+// 100 graphs of scales 10-12); with IPT = 1 single edges.  A claim is an atomicOr on the visited
 // bitmap -- the block's own shared bitmap, or, for a graph shared by a cluster
 // (CL), the cluster's bitmap in global memory, with the shared bitmap kept as a
 // filter of already visited vertices; a lane's claims are in flight together.
@@ -103,7 +105,8 @@ __device__ __forceinline__ unsigned long long multi_level(
     uint32_t tile0, uint32_t tstride, uint32_t *s_bitmap, uint32_t *gb, uint32_t *ctr,
     MultiTile<B> &s) {
   constexpr int NW = B / 32;
-  constexpr bool kChunks = IPT == 4;
+  constexpr bool kChunks = IPT >= 2;
+  constexpr int kSlots = kChunks ? 4 : IPT;  // edges per lane
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t lt_mask = (1u << lane) - 1u;
   // chunks are counted from the 16-byte boundary at or below ix
@@ -149,7 +152,7 @@ __device__ __forceinline__ unsigned long long multi_level(
       }
       uint32_t cur = lo;
       for (uint32_t base = w0; base < w1; base += kChunks ? 32u : 32u * IPT) {
-        uint32_t nb[IPT], on = 0;  // targets; bit u: slot u holds one
+        uint32_t nb[kSlots], on = 0;  // targets; bit u: slot u holds one
         if constexpr (kChunks) {
           const uint32_t x = base + lane;
           const uint32_t j = cur + 1u + lane;
@@ -191,9 +194,9 @@ __device__ __forceinline__ unsigned long long multi_level(
             on |= addr[u] != kFull ? 1u << u : 0u;
           }
         }
-        uint32_t old[IPT];
+        uint32_t old[kSlots];
 #pragma unroll
-        for (int u = 0; u < IPT; u++) {
+        for (int u = 0; u < kSlots; u++) {
           const uint32_t w = nb[u] >> 5, bit = 1u << (nb[u] & 31u);
           old[u] = kFull;  // visited
           if (((on >> u) & 1u) && !(s_bitmap[w] & bit)) {
@@ -201,9 +204,9 @@ __device__ __forceinline__ unsigned long long multi_level(
             if (CL) atomicOr(s_bitmap + w, bit);
           }
         }
-        uint32_t push[IPT], num = 0;
+        uint32_t push[kSlots], num = 0;
 #pragma unroll
-        for (int u = 0; u < IPT; u++) {
+        for (int u = 0; u < kSlots; u++) {
           const bool mine = !((old[u] >> (nb[u] & 31u)) & 1u);
           if (mine) lv[nb[u]] = lvl + 1;
           push[u] = __ballot_sync(kFull, mine && nb[u] < n_rows);
@@ -214,7 +217,7 @@ __device__ __forceinline__ unsigned long long multi_level(
         if (lane == 0) at = atomicAdd(ctr, num);
         at = __shfl_sync(kFull, at, 0);
 #pragma unroll
-        for (int u = 0; u < IPT; u++) {
+        for (int u = 0; u < kSlots; u++) {
           if ((push[u] >> lane) & 1u) qn[at + __popc(push[u] & lt_mask)] = nb[u];
           at += __popc(push[u]);
         }
@@ -472,10 +475,14 @@ static bfs_status multi_prepare(bfs_multi *m, int cfg, int32_t *levels_dev) {
   uint32_t n_big = 0;
   if (c.cluster > 1) {
     grid = std::max(c.cluster, grid / c.cluster * c.cluster);
-    // a graph is shared by a cluster when its edges exceed a quarter of
-    // `cluster` blocks' fair share of the batch's edges
-    for (uint32_t i = 0; i < m->n_graphs; i++)
-      if ((double)m->order_nnz[i] * grid * 4.0 >= (double)m->total_edges * c.cluster) n_big = i + 1;
+    // a graph is shared by a cluster when its edges exceed `cluster` blocks'
+    // fair share of the batch's edges, or a quarter of it where that is enough
+    // work for a cluster's barriers (169 graphs of 13 K to 26 K edges: 98 us
+    // with the whole share, 107 with a quarter)
+    for (uint32_t i = 0; i < m->n_graphs; i++) {
+      const double shares = (double)m->order_nnz[i] * grid / ((double)m->total_edges * c.cluster);
+      if (shares >= 1.0 || (shares >= 0.25 && m->order_nnz[i] >= kShareEdges)) n_big = i + 1;
+    }
     const size_t n_clusters = (size_t)grid / c.cluster;
     if (m->gbits_words < n_clusters * words) {
       cudaFree(m->d_gbits);

@@ -243,8 +243,8 @@ bfs_status bfs_multi_free(bfs_multi *m);
  * n_cols of the graphs before it). */
 bfs_status bfs_multi_level_offset(const bfs_multi *m, uint32_t graph, uint64_t *offset);
 /* levels_dev: sum of n_cols int32 (device).  block 128/256/512, ipt 1/2/4
- * (warp rounds in flight per lane).  edges_count_out: n_graphs (host,
- * optional); device_ms: CUDA-event time of the launch (optional). */
+ * (1: single edges, 2 and 4: a 16-byte chunk of edges per lane and round).
+ * edges_count_out: n_graphs (host, optional); device_ms: CUDA-event time of the launch (optional). */
 bfs_status bfs_multi_run(bfs_multi *m, const uint32_t *roots, int32_t block, int32_t ipt,
                          int32_t *levels_dev, uint64_t *edges_count_out, double *device_ms);
 /* Times every (block, ipt) combination on this batch (best of reps) and
