@@ -482,9 +482,10 @@ __device__ __forceinline__ int32_t sext_byte(uint32_t x, int i) {
 // Stores the rows of up to 32 roots (nl of them, `row` the first) for the
 // vertices v + 32 i (i < kXv) of a warp's lanes: kXv 128-byte segments of a row
 // follow each other.
-constexpr int kXv = 4;
 constexpr int kXl = 4;  // history levels loaded together
 constexpr int kXb = 3;  // blocks per SM
+
+template <int kXv>
 __device__ __forceinline__ void ms_store_rows(int32_t *__restrict__ row, size_t n, uint64_t v,
                                               uint32_t nl, const uint32_t (&r)[kXv],
                                               const uint32_t (&b0)[kXv], const uint32_t (&b1)[kXv],
@@ -513,8 +514,66 @@ __device__ __forceinline__ void ms_store_rows(int32_t *__restrict__ row, size_t 
   }
 }
 
+// Writes every root's row from the history levels up to lmax.
+template <int kXv>
+__device__ __forceinline__ void ms_expand_rows(const MsState *__restrict__ st, uint32_t lmax,
+                                               uint64_t gwarp, uint64_t warps) {
+  const uint64_t n = st->n_cols;
+  const uint32_t nl = st->n_lanes, lane = threadIdx.x & 31u;
+  int32_t *__restrict__ level = st->level;
+  const uint32_t *__restrict__ pinv = st->pinv;
+  const uint32_t *__restrict__ moved = st->moved;
+  // an item: 32 kXv vertices and 32 roots (one half of the masks)
+  const uint32_t halves = nl > 32u ? 2u : 1u;
+  const uint32_t *__restrict__ hist = reinterpret_cast<const uint32_t *>(st->hist);
+  const uint64_t items = (n + 32u * kXv - 1u) / (32u * kXv) * halves;
+  for (uint64_t it = gwarp; it < items; it += warps) {
+    const uint32_t half = halves == 2u ? (uint32_t)it & 1u : 0u;
+    const uint64_t ov = it / halves * (32u * kXv) + lane;  // original ids ov + 32 i
+    uint32_t r[kXv], p0[kXv], p1[kXv], p2[kXv], p3[kXv];
+    const uint32_t *at[kXv];
+#pragma unroll
+    for (int i = 0; i < kXv; i++) {
+      const uint64_t o = ov + 32u * i;
+      // internal id whose masks belong to it (moved ids only differ)
+      uint64_t v = o;
+      if (moved && o < n && ((moved[o >> 5] >> (o & 31u)) & 1u)) v = pinv[o];
+      at[i] = hist + 2u * v + half;
+      r[i] = p0[i] = p1[i] = p2[i] = p3[i] = 0u;
+    }
+    // within levels L0 .. L0 + 3 (L0 a multiple of 4) bits 0 and 1 of the
+    // level are those of k, bits 2 and 3 those of L0
+    for (uint32_t L0 = 0; L0 <= lmax; L0 += kXl) {
+      uint32_t m[kXl][kXv];
+#pragma unroll
+      for (int k = 0; k < kXl; k++)
+#pragma unroll
+        for (int i = 0; i < kXv; i++)
+          m[k][i] = (L0 + k <= lmax && ov + 32u * i < n)
+                        ? at[i][(size_t)(L0 + k) * 2u * n] : 0u;
+#pragma unroll
+      for (int i = 0; i < kXv; i++) {
+#pragma unroll
+        for (int h = 0; h < kXl; h += 4) {
+          const uint32_t all4 = m[h][i] | m[h + 1][i] | m[h + 2][i] | m[h + 3][i];
+          r[i] |= all4;
+          p0[i] |= m[h + 1][i] | m[h + 3][i];
+          p1[i] |= m[h + 2][i] | m[h + 3][i];
+          if ((L0 + h) & 4u) p2[i] |= all4;
+          if ((L0 + h) & 8u) p3[i] |= all4;
+        }
+      }
+    }
+    ms_store_rows<kXv>(level + (size_t)(half * 32u) * n, n, ov, min(32u, nl - half * 32u), r, p0, p1,
+                  p2, p3);
+  }
+}
+
+// Vertices from which a lane takes four.
+constexpr uint32_t kXvVertices = 1u << 17;
+
 __global__ void __launch_bounds__(kMsBlock, kXb) ms_expand_kernel(MsState *__restrict__ st,
-                                                                int final) {
+                                                                  int final) {
   static_assert(kHistLevels <= 16, "levels must fit four bit planes");
   __shared__ unsigned long long s_edges[kLanes];
   __shared__ unsigned long long s_common;
@@ -535,50 +594,11 @@ __global__ void __launch_bounds__(kMsBlock, kXb) ms_expand_kernel(MsState *__res
   const uint64_t gwarp = ((uint64_t)blockIdx.x * kMsBlock + threadIdx.x) >> 5;
   const uint64_t warps = (uint64_t)gridDim.x * (kMsBlock / 32);
   if (expand) {
-    // an item: 32 kXv vertices and 32 roots (one half of the masks)
-    const uint32_t halves = nl > 32u ? 2u : 1u;
-    const uint32_t *__restrict__ hist = reinterpret_cast<const uint32_t *>(st->hist);
-    const uint64_t items = (n + 32u * kXv - 1u) / (32u * kXv) * halves;
-    for (uint64_t it = gwarp; it < items; it += warps) {
-      const uint32_t half = halves == 2u ? (uint32_t)it & 1u : 0u;
-      const uint64_t ov = it / halves * (32u * kXv) + lane;  // original ids ov + 32 i
-      uint32_t r[kXv], p0[kXv], p1[kXv], p2[kXv], p3[kXv];
-      const uint32_t *at[kXv];
-#pragma unroll
-      for (int i = 0; i < kXv; i++) {
-        const uint64_t o = ov + 32u * i;
-        // internal id whose masks belong to it (moved ids only differ)
-        uint64_t v = o;
-        if (moved && o < n && ((moved[o >> 5] >> (o & 31u)) & 1u)) v = pinv[o];
-        at[i] = hist + 2u * v + half;
-        r[i] = p0[i] = p1[i] = p2[i] = p3[i] = 0u;
-      }
-      // within levels L0 .. L0 + 3 (L0 a multiple of 4) bits 0 and 1 of the
-      // level are those of k, bits 2 and 3 those of L0
-      for (uint32_t L0 = 0; L0 <= lmax; L0 += kXl) {
-        uint32_t m[kXl][kXv];
-#pragma unroll
-        for (int k = 0; k < kXl; k++)
-#pragma unroll
-          for (int i = 0; i < kXv; i++)
-            m[k][i] = (L0 + k <= lmax && ov + 32u * i < n)
-                          ? at[i][(size_t)(L0 + k) * 2u * n] : 0u;
-#pragma unroll
-        for (int i = 0; i < kXv; i++) {
-#pragma unroll
-          for (int h = 0; h < kXl; h += 4) {
-            const uint32_t all4 = m[h][i] | m[h + 1][i] | m[h + 2][i] | m[h + 3][i];
-            r[i] |= all4;
-            p0[i] |= m[h + 1][i] | m[h + 3][i];
-            p1[i] |= m[h + 2][i] | m[h + 3][i];
-            if ((L0 + h) & 4u) p2[i] |= all4;
-            if ((L0 + h) & 8u) p3[i] |= all4;
-          }
-        }
-      }
-      ms_store_rows(level + (size_t)(half * 32u) * n, n, ov, min(32u, nl - half * 32u), r, p0, p1,
-                    p2, p3);
-    }
+    // with few vertices the warps that one vertex per lane gives matter more
+    // than the runs of a row (R-MAT scale 12, 4 roots: 178 us
+    // per call instead of 184)
+    if (n >= kXvVertices) ms_expand_rows<4>(st, lmax, gwarp, warps);
+    else ms_expand_rows<1>(st, lmax, gwarp, warps);
   }
   if (!final) return;
   if (threadIdx.x < kLanes) s_edges[threadIdx.x] = 0;
