@@ -16,8 +16,8 @@
 //             boundaries plus popc instead of a per-edge binary search
 //             (:448-464, :336-346).  Visiting tests one bit of a visited
 //             bitmap (n/8 bytes, pinned in L2 through an access-policy window)
-//             with a plain load and only then claims it with atomicOr, instead
-//             of byte masks.
+//             with a plain load and only then claims it with a reduction,
+//             instead of byte masks.
 //   levelgen  scans the bitmap words (n/32, not n bytes): new = vis & ~prev.
 //             Blocks claim spans of words from a counter, write the new
 //             levels a bitmap word (one 32-byte sector of one-byte working
