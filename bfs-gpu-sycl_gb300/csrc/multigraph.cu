@@ -487,12 +487,14 @@ static bfs_status multi_prepare(bfs_multi *m, int cfg, int32_t *levels_dev) {
     if (m->gbits_words < n_clusters * words) {
       cudaFree(m->d_gbits);
       m->d_gbits = nullptr;
+      m->gbits_words = 0;  // stays so if the allocation fails
       GK(dev_malloc(&m->d_gbits, sizeof(uint32_t) * n_clusters * words));
       m->gbits_words = n_clusters * words;
     }
     if (m->gcnt_words < n_clusters * 4) {
       cudaFree(m->d_gcnt);
       m->d_gcnt = nullptr;
+      m->gcnt_words = 0;
       GK(dev_malloc(&m->d_gcnt, sizeof(uint32_t) * n_clusters * 4));
       m->gcnt_words = n_clusters * 4;
     }
