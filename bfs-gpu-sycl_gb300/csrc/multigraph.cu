@@ -427,6 +427,7 @@ struct bfs_multi {
   uint32_t *d_gbits = nullptr, *d_gcnt = nullptr;  // cluster bitmaps and counters
   size_t gbits_words = 0, gcnt_words = 0;
   std::vector<uint64_t> order_nnz;                   // edge counts in claim order
+  uint64_t sizes_hash = 0;                           // of all graphs' sizes, in claim order
   uint32_t n_big = 0;
   MultiDesc *d_descs = nullptr;
   unsigned long long *d_edges = nullptr;
@@ -579,7 +580,13 @@ bfs_status bfs_multi_create(uint32_t n_graphs, const uint32_t *const *indptrs,
   std::stable_sort(order.begin(), order.end(),
                    [&](uint32_t a, uint32_t b) { return nnz[a] > nnz[b]; });
   m->order_nnz.resize(n_graphs);
-  for (uint32_t i = 0; i < n_graphs; i++) m->order_nnz[i] = nnz[order[i]];
+  m->sizes_hash = 14695981039346656037ull;  // FNV-1a over words
+  for (uint32_t i = 0; i < n_graphs; i++) {
+    const uint32_t g = order[i];
+    m->order_nnz[i] = nnz[g];
+    for (uint64_t x : {nnz[g], (uint64_t)n_cols[g], (uint64_t)n_rows[g]})
+      m->sizes_hash = (m->sizes_hash ^ x) * 1099511628211ull;
+  }
   bfs_status rc = BFS_OK;
   std::vector<uint32_t> hip(vb), hix(eb ? eb : 1);
   for (uint32_t g = 0; g < n_graphs; g++) {
@@ -717,9 +724,14 @@ bfs_status bfs_multi_run_ex(bfs_multi *m, const uint32_t *roots, int32_t block, 
 
 }  // extern "C"
 
+// Raised whenever a kernel or the rule for sharing graphs changes: a choice
+// cached before was timed on other code.
+constexpr int kMultiRevision = 3;
+
 // Times configurations [0, n_cfg) on the batch (best of reps after a warm-up
 // run that also captures the launch) and returns the fastest; a cache file
-// keeps the choice per GPU, batch shape and configuration set.
+// keeps the choice per GPU, kernel revision, configuration set and sizes of the
+// batch's graphs (batches of equal totals differ in what clusters share).
 static bfs_status multi_autotune(bfs_multi *m, const uint32_t *roots, int32_t *levels_dev,
                                  int32_t reps, const char *cache_path, int n_cfg, int *best_out,
                                  float *times_ms) {
@@ -729,7 +741,8 @@ static bfs_status multi_autotune(bfs_multi *m, const uint32_t *roots, int32_t *l
   GK(cudaGetDeviceProperties(&prop, m->device));
   std::ostringstream key;
   key << prop.name << "|sm" << prop.multiProcessorCount << "|g" << m->n_graphs << "|v"
-      << m->total_cols << "|e" << m->total_edges << "|c" << n_cfg;
+      << m->total_cols << "|e" << m->total_edges << "|c" << n_cfg << "|h" << std::hex
+      << m->sizes_hash << "|r" << std::dec << kMultiRevision;
   if (cache_path && cache_path[0]) {
     std::ifstream in(cache_path);
     std::string line;

@@ -248,8 +248,9 @@ bfs_status bfs_multi_level_offset(const bfs_multi *m, uint32_t graph, uint64_t *
 bfs_status bfs_multi_run(bfs_multi *m, const uint32_t *roots, int32_t block, int32_t ipt,
                          int32_t *levels_dev, uint64_t *edges_count_out, double *device_ms);
 /* Times every (block, ipt) combination on this batch (best of reps) and
- * returns the fastest.  With cache_path, a previous result for the same GPU
- * and batch shape is reused and a new one is appended.  times_ms (optional)
+ * returns the fastest.  With cache_path, a previous result for the same GPU,
+ * the same revision of the kernels and graphs of the same sizes is reused, and
+ * a new one is appended.  times_ms (optional)
  * receives the 9 timings, block-major (-1 when taken from the cache). */
 bfs_status bfs_multi_autotune(bfs_multi *m, const uint32_t *roots, int32_t *levels_dev,
                               int32_t reps, const char *cache_path, int32_t *best_block,

@@ -1,5 +1,5 @@
 """What a batch of many graphs keeps between calls: the clusters' bitmaps after
-an allocation that failed."""
+an allocation that failed, and the file of tuned configurations."""
 import numpy as np
 import pytest
 
@@ -43,3 +43,39 @@ def test_cluster_bitmaps_after_a_failed_allocation(B, O, monkeypatch):
     monkeypatch.delenv(HOOK)
     check(O, batch, graphs, roots, out, (256, 2, 2))
     batch.free()
+
+
+def uniform(B, n, m, seed):
+    rng = np.random.default_rng(seed)
+    src = np.sort(rng.integers(0, n, m))
+    indptr = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))])
+    return B.Csc(indptr, rng.integers(0, n, m))
+
+
+@pytest.mark.parametrize("clusters", [False, True])
+def test_tuned_configuration_is_reused_only_for_its_kernels_and_sizes(B, tmp_path, clusters):
+    torch = torch_cuda()
+    path = tmp_path / "tuned.tsv"
+
+    def tune(graphs):
+        batch = B.MultiBatch(graphs)
+        out = torch.empty(batch.total_cols, dtype=torch.int32, device="cuda")
+        best, times = batch.autotune([0] * len(graphs), out.data_ptr(), reps=1,
+                                     cache_path=str(path), clusters=clusters)
+        batch.free()
+        return best, all(t > 0 for t in times)
+
+    even = [uniform(B, 2000, 8000, 1), uniform(B, 2000, 8000, 2)]
+    best, timed = tune(even)
+    assert timed
+    assert tune(even) == (best, False)  # from the file
+    # equal numbers of graphs, vertices and edges, other sizes
+    uneven = [uniform(B, 1000, 4000, 3), uniform(B, 3000, 12000, 4)]
+    assert tune(uneven)[1]
+    assert not tune(uneven)[1] and not tune(even)[1]
+    # lines of another revision of the kernels, and of the key without one
+    key, cfg = path.read_text().splitlines()[0].split("\t")
+    head, sep, rev = key.rpartition("|r")
+    assert sep
+    path.write_text(f"{head}|r{int(rev) + 1}\t{cfg}\n{head}\t{cfg}\n{head.split('|h')[0]}\t{cfg}\n")
+    assert tune(even)[1]
