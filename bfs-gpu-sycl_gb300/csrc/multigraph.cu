@@ -9,15 +9,16 @@
 // graph on its own, with the visited bitmap in shared memory and __syncthreads
 // as the level barrier.  Within a level the block uses the LLB form: a block
 // exclusive scan of a tile's degrees, the tile's edges split evenly over the
-// warps, owners resolved per warp round (bfs_internal / device_util), IPT
-// rounds in flight per lane.  A claim is an atomicOr on the shared bitmap; the
+// warps, owners resolved per warp round (bfs_internal / device_util), a 16-byte
+// chunk of edges or one edge per lane.  A claim is an atomicOr on the shared bitmap; the
 // claiming thread writes the level and appends the vertex to the next queue
 // (vertices >= n_rows get a level but are not queued; those without out-edges
 // are dropped when the next level loads their offsets).
 //
-// Block size (128/256/512) and items per thread (1/2/4 rounds per lane) come
-// from an autotuner that times every combination on the batch and caches the
-// choice per GPU and batch shape.  The launch (work-counter reset, level fill,
+// Block size (128/256/512), the form of a round (items per thread: 1 for single
+// edges, 2 or 4 for chunks) and the cluster size come from an autotuner that
+// times every combination on the batch and caches the choice per GPU, kernel
+// revision and graph sizes.  The launch (work-counter reset, level fill,
 // persistent kernel) is captured once into a CUDA graph and replayed.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -80,10 +81,10 @@ struct MultiTile {
 // One level of one graph over tiles tile0, tile0 + tstride, ... of B
 // frontier entries (LLB form): block exclusive scan over the tile, entries
 // without edges dropped, the tile's edges split evenly over the warps, owners
-// resolved per warp round.  With IPT of 2 or more a round deals 16-byte chunks
+// resolved per warp round.  With CHUNKS a round deals 16-byte chunks
 // of the edge array, one per lane -- four edges in flight for one owner
-// resolution (two rounds of single edges at IPT = 2 took 100 us instead of 74 on
-// 100 graphs of scales 10-12); with IPT = 1 single edges.  A claim is an atomicOr on the visited
+// resolution (two rounds of single edges took 100 us instead of 74 on 100 graphs
+// of scales 10-12); otherwise single edges.  A claim is an atomicOr on the visited
 // bitmap -- the block's own shared bitmap, or, for a graph shared by a cluster
 // (CL), the cluster's bitmap in global memory, with the shared bitmap kept as a
 // filter of already visited vertices; a lane's claims are in flight together.
@@ -98,19 +99,18 @@ struct MultiTile {
 // instead of a whole one as the limit for sharing a graph 0.93 -> 0.78 (half,
 // eighth, sixteenth: 0.79, 0.78, 0.81); chunks 0.78 -> 0.59.  Registers for 2
 // or 3 blocks of 512 threads per SM instead of 4: 0.80, 0.76.
-template <int B, int IPT, bool CL>
+template <int B, bool CHUNKS, bool CL>
 __device__ __forceinline__ unsigned long long multi_level(
     const uint32_t *__restrict__ ip, const uint32_t *__restrict__ ix, int32_t *lv,
     uint32_t n_rows, const uint32_t *qc, uint32_t *qn, uint32_t F, int32_t lvl,
     uint32_t tile0, uint32_t tstride, uint32_t *s_bitmap, uint32_t *gb, uint32_t *ctr,
     MultiTile<B> &s) {
   constexpr int NW = B / 32;
-  constexpr bool kChunks = IPT >= 2;
-  constexpr int kSlots = kChunks ? 4 : IPT;  // edges per lane
+  constexpr int kSlots = CHUNKS ? 4 : 1;  // edges per lane
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   const uint32_t lt_mask = (1u << lane) - 1u;
   // chunks are counted from the 16-byte boundary at or below ix
-  const uint32_t eoff = kChunks ? (uint32_t)((reinterpret_cast<uintptr_t>(ix) & 15u) >> 2) : 0u;
+  const uint32_t eoff = CHUNKS ? (uint32_t)((reinterpret_cast<uintptr_t>(ix) & 15u) >> 2) : 0u;
   const uint4 *__restrict__ ix4 = reinterpret_cast<const uint4 *>(ix - eoff);
   unsigned long long edges = 0;
   for (uint32_t tile = tile0; tile < F; tile += tstride) {
@@ -123,7 +123,7 @@ __device__ __forceinline__ unsigned long long multi_level(
       beg += eoff;
     }
     edges += deg;
-    const uint32_t units = kChunks ? edge_chunks(beg, deg, 0u) : deg;
+    const uint32_t units = CHUNKS ? edge_chunks(beg, deg, 0u) : deg;
     const uint32_t incl = warp_incl_scan(units, lane);
     const uint32_t has = __ballot_sync(kFull, deg > 0u);
     if (lane == 31) s.wsum[warp] = make_uint2(incl, __popc(has));
@@ -137,7 +137,7 @@ __device__ __forceinline__ unsigned long long multi_level(
       const uint32_t i = (warp ? cprev : 0u) + __popc(has & lt_mask);
       s.off[i] = (warp ? uprev : 0u) + incl - units;
       s.beg[i] = beg;
-      if (kChunks) s.deg[i] = deg;
+      if (CHUNKS) s.deg[i] = deg;
     }
     if (threadIdx.x == 0) s.off[m] = total;
     __syncthreads();
@@ -151,9 +151,9 @@ __device__ __forceinline__ unsigned long long multi_level(
         if (s.off[mid] <= w0) lo = mid; else hi = mid;
       }
       uint32_t cur = lo;
-      for (uint32_t base = w0; base < w1; base += kChunks ? 32u : 32u * IPT) {
+      for (uint32_t base = w0; base < w1; base += 32u) {
         uint32_t nb[kSlots], on = 0;  // targets; bit u: slot u holds one
-        if constexpr (kChunks) {
+        if constexpr (CHUNKS) {
           const uint32_t x = base + lane;
           const uint32_t j = cur + 1u + lane;
           const uint32_t bnd = j <= m ? s.off[j] : kFull;
@@ -175,24 +175,15 @@ __device__ __forceinline__ unsigned long long multi_level(
           nb[2] = q.z;
           nb[3] = q.w;
         } else {
-          uint32_t addr[IPT];
-#pragma unroll
-          for (int u = 0; u < IPT; u++) {
-            const uint32_t rb = base + 32u * u;
-            const uint32_t e = rb + lane;
-            const uint32_t j = cur + 1u + lane;
-            const uint32_t bnd = j <= m ? s.off[j] : kFull;
-            const uint32_t starts = __reduce_or_sync(kFull, bit_or_zero(bnd - rb));
-            const uint32_t o = cur + __popc(starts & ((2u << lane) - 1u));
-            addr[u] = (e < w1) ? s.beg[o] + (e - s.off[o]) : kFull;
-            cur += __popc(starts);
-            if (cur >= m) cur = m - 1;  // only reached past w1
-          }
-#pragma unroll
-          for (int u = 0; u < IPT; u++) {
-            nb[u] = addr[u] != kFull ? ix[addr[u]] : 0u;
-            on |= addr[u] != kFull ? 1u << u : 0u;
-          }
+          const uint32_t e = base + lane;
+          const uint32_t j = cur + 1u + lane;
+          const uint32_t bnd = j <= m ? s.off[j] : kFull;
+          const uint32_t starts = __reduce_or_sync(kFull, bit_or_zero(bnd - base));
+          const uint32_t o = cur + __popc(starts & ((2u << lane) - 1u));
+          cur += __popc(starts);
+          if (cur >= m) cur = m - 1;  // only reached past w1
+          on = e < w1 ? 1u : 0u;
+          nb[0] = e < w1 ? ix[s.beg[o] + (e - s.off[o])] : 0u;
         }
         uint32_t old[kSlots];
 #pragma unroll
@@ -237,7 +228,7 @@ __device__ __forceinline__ void add_edges(unsigned long long *out, unsigned long
 
 // A complete BFS of one graph by one block, the visited bitmap in shared
 // memory and __syncthreads as the level barrier.
-template <int B, int IPT>
+template <int B, bool CHUNKS>
 __device__ __forceinline__ void multi_graph_block(const MultiArgs &a, uint32_t gi,
                                                   uint32_t *s_bitmap, MultiTile<B> &s) {
   const MultiDesc d = a.descs[a.order[gi]];
@@ -266,7 +257,7 @@ __device__ __forceinline__ void multi_graph_block(const MultiArgs &a, uint32_t g
     __syncthreads();
     if (threadIdx.x == 0) s.next = 0;
     __syncthreads();
-    edges += multi_level<B, IPT, false>(ip, ix, lv, d.n_rows, qc, qn, F, lvl, 0u, B, s_bitmap,
+    edges += multi_level<B, CHUNKS, false>(ip, ix, lv, d.n_rows, qc, qn, F, lvl, 0u, B, s_bitmap,
                                         nullptr, &s.next, s);
     __syncthreads();
     F = s.next;
@@ -279,7 +270,7 @@ __device__ __forceinline__ void multi_graph_block(const MultiArgs &a, uint32_t g
 }
 
 // Graphs claimed one per block from a work counter (largest first).
-template <int B, int IPT>
+template <int B, bool CHUNKS>
 __device__ __forceinline__ void multi_small_graphs(const MultiArgs &a, uint32_t *s_bitmap,
                                                    MultiTile<B> &s) {
   for (;;) {
@@ -287,16 +278,16 @@ __device__ __forceinline__ void multi_small_graphs(const MultiArgs &a, uint32_t 
     __syncthreads();
     const uint32_t gi = s.graph;
     if (gi >= a.n_graphs) break;
-    multi_graph_block<B, IPT>(a, gi, s_bitmap, s);
+    multi_graph_block<B, CHUNKS>(a, gi, s_bitmap, s);
     __syncthreads();
   }
 }
 
-template <int B, int IPT>
+template <int B, bool CHUNKS>
 __global__ void __launch_bounds__(B, 2048 / B) multi_bfs_kernel(MultiArgs a) {
   extern __shared__ uint32_t s_bitmap[];
   __shared__ MultiTile<B> s;
-  multi_small_graphs<B, IPT>(a, s_bitmap, s);
+  multi_small_graphs<B, CHUNKS>(a, s_bitmap, s);
 }
 
 // Clusters of C blocks first share the largest graphs (order[0, n_big)): a
@@ -308,7 +299,7 @@ __global__ void __launch_bounds__(B, 2048 / B) multi_bfs_kernel(MultiArgs a) {
 // counters in global memory.  Then every block takes small graphs on its
 // own.  Each frontier entry is expanded by exactly one block, so the edge
 // counts stay exact.
-template <int B, int IPT, int C>
+template <int B, int C>
 __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(B, 2048 / B)
     multi_bfs_cluster_kernel(MultiArgs a) {
   extern __shared__ uint32_t s_bitmap[];
@@ -357,7 +348,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(B, 2048 / B)
       uint32_t *qc = (lvl & 1) ? cq1 : cq0;
       uint32_t *qn = (lvl & 1) ? cq0 : cq1;
       uint32_t *ctr = cnt + (lvl + 1) % 3;
-      edges += multi_level<B, IPT, true>(ip, ix, lv, d.n_rows, qc, qn, F, lvl, rank * B, C * B,
+      edges += multi_level<B, true, true>(ip, ix, lv, d.n_rows, qc, qn, F, lvl, rank * B, C * B,
                                          s_bitmap, gb, ctr, s);
       cl.sync();
       const uint32_t fn = __ldcg(ctr);
@@ -379,7 +370,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(B, 2048 / B)
     add_edges(a.edges_out + a.order[gi], edges);
     cl.sync();  // queues, counters and bitmap are free for the cluster's next graph
   }
-  multi_small_graphs<B, IPT>(a, s_bitmap, s);
+  multi_small_graphs<B, true>(a, s_bitmap, s);
 }
 
 __global__ void multi_fill_kernel(int32_t *levels, uint64_t n) {
@@ -395,18 +386,20 @@ struct MultiConfig {
   MultiKernel fn;
 };
 
+// ipt 2 and 4 both name the chunk form.
 static const MultiConfig kMultiConfigs[] = {
-    {128, 1, 1, multi_bfs_kernel<128, 1>}, {128, 2, 1, multi_bfs_kernel<128, 2>},
-    {128, 4, 1, multi_bfs_kernel<128, 4>}, {256, 1, 1, multi_bfs_kernel<256, 1>},
-    {256, 2, 1, multi_bfs_kernel<256, 2>}, {256, 4, 1, multi_bfs_kernel<256, 4>},
-    {512, 1, 1, multi_bfs_kernel<512, 1>}, {512, 2, 1, multi_bfs_kernel<512, 2>},
-    {512, 4, 1, multi_bfs_kernel<512, 4>},
-    {256, 2, 2, multi_bfs_cluster_kernel<256, 2, 2>}, {256, 4, 2, multi_bfs_cluster_kernel<256, 4, 2>},
-    {512, 2, 2, multi_bfs_cluster_kernel<512, 2, 2>}, {512, 4, 2, multi_bfs_cluster_kernel<512, 4, 2>},
-    {256, 2, 4, multi_bfs_cluster_kernel<256, 2, 4>}, {256, 4, 4, multi_bfs_cluster_kernel<256, 4, 4>},
-    {512, 2, 4, multi_bfs_cluster_kernel<512, 2, 4>}, {512, 4, 4, multi_bfs_cluster_kernel<512, 4, 4>},
-    {256, 2, 8, multi_bfs_cluster_kernel<256, 2, 8>}, {256, 4, 8, multi_bfs_cluster_kernel<256, 4, 8>},
-    {512, 2, 8, multi_bfs_cluster_kernel<512, 2, 8>}, {512, 4, 8, multi_bfs_cluster_kernel<512, 4, 8>},
+    {128, 1, 1, multi_bfs_kernel<128, false>}, {128, 2, 1, multi_bfs_kernel<128, true>},
+    {128, 4, 1, multi_bfs_kernel<128, true>},
+    {256, 1, 1, multi_bfs_kernel<256, false>}, {256, 2, 1, multi_bfs_kernel<256, true>},
+    {256, 4, 1, multi_bfs_kernel<256, true>},
+    {512, 1, 1, multi_bfs_kernel<512, false>}, {512, 2, 1, multi_bfs_kernel<512, true>},
+    {512, 4, 1, multi_bfs_kernel<512, true>},
+    {256, 2, 2, multi_bfs_cluster_kernel<256, 2>}, {256, 4, 2, multi_bfs_cluster_kernel<256, 2>},
+    {512, 2, 2, multi_bfs_cluster_kernel<512, 2>}, {512, 4, 2, multi_bfs_cluster_kernel<512, 2>},
+    {256, 2, 4, multi_bfs_cluster_kernel<256, 4>}, {256, 4, 4, multi_bfs_cluster_kernel<256, 4>},
+    {512, 2, 4, multi_bfs_cluster_kernel<512, 4>}, {512, 4, 4, multi_bfs_cluster_kernel<512, 4>},
+    {256, 2, 8, multi_bfs_cluster_kernel<256, 8>}, {256, 4, 8, multi_bfs_cluster_kernel<256, 8>},
+    {512, 2, 8, multi_bfs_cluster_kernel<512, 8>}, {512, 4, 8, multi_bfs_cluster_kernel<512, 8>},
 };
 constexpr int kNumMultiConfigs = sizeof(kMultiConfigs) / sizeof(kMultiConfigs[0]);
 constexpr int kNumSingleConfigs = 9;  // the first 9: one block per graph
@@ -728,7 +721,7 @@ bfs_status bfs_multi_run_ex(bfs_multi *m, const uint32_t *roots, int32_t block, 
 // cached before was timed on other code.
 constexpr int kMultiRevision = 3;
 
-// Times configurations [0, n_cfg) on the batch (best of reps after a warm-up
+// Times the kernels of configurations [0, n_cfg) on the batch (best of reps after a warm-up
 // run that also captures the launch) and returns the fastest; a cache file
 // keeps the choice per GPU, kernel revision, configuration set and sizes of the
 // batch's graphs (batches of equal totals differ in what clusters share).
@@ -765,6 +758,12 @@ static bfs_status multi_autotune(bfs_multi *m, const uint32_t *roots, int32_t *l
   float best_ms = 1e30f;
   for (int i = 0; i < n_cfg; i++) {
     const MultiConfig &c = kMultiConfigs[i];
+    int same = 0;  // a configuration before it with the same kernel is not timed again
+    while (kMultiConfigs[same].fn != c.fn) same++;
+    if (same < i) {
+      if (times_ms) times_ms[i] = times_ms[same];
+      continue;
+    }
     double t = 0.0, mn = 1e30;
     bfs_status rc = bfs_multi_run_ex(m, roots, c.block, c.ipt, c.cluster, levels_dev, nullptr,
                                      &t);  // warm-up + capture

@@ -1,5 +1,6 @@
 """What a batch of many graphs keeps between calls: the clusters' bitmaps after
-an allocation that failed, and the file of tuned configurations."""
+an allocation that failed, and the file of tuned configurations; each kernel is
+timed once."""
 import numpy as np
 import pytest
 
@@ -79,3 +80,19 @@ def test_tuned_configuration_is_reused_only_for_its_kernels_and_sizes(B, tmp_pat
     assert sep
     path.write_text(f"{head}|r{int(rev) + 1}\t{cfg}\n{head}\t{cfg}\n{head.split('|h')[0]}\t{cfg}\n")
     assert tune(even)[1]
+
+
+def test_each_kernel_is_timed_once(B):
+    """Items per thread 2 and 4 name the same kernel: one time for both, and the
+    choice is not left to noise between them."""
+    torch = torch_cuda()
+    batch = B.MultiBatch([uniform(B, 3000, 20000, s) for s in range(3)])
+    out = torch.empty(batch.total_cols, dtype=torch.int32, device="cuda")
+    for clusters in (False, True):
+        best, times = batch.autotune([0, 1, 2], out.data_ptr(), reps=3, clusters=clusters)
+        configs = B.MULTI_CONFIGS_ALL[:len(times)]
+        t = dict(zip(configs, times))
+        assert all(x > 0 for x in times)
+        assert all(t[b, 2, c] == t[b, 4, c] for b, p, c in configs if p == 4)
+        assert best[1] != 4 and t[(best + (1,))[:3]] == min(times)
+    batch.free()
