@@ -634,19 +634,24 @@ bfs_status run_device_impl(bfs_graph *g, uint32_t root, const bfs_options *opts_
     g->prof_gen = stats->level_gen_ms;
     clear_level_times(stats);
   }
-  bfs_status hrc = ensure_hub(g);
-  if (hrc != BFS_OK) return hrc;
+  // The layout serves plans that run GLB levels (fixed GLB arms, the learned
+  // schedule, the per-level recorder) and is built by the first of them.  Fixed
+  // LLB and SLB search the graph as it is given.  The layout's numbering gives
+  // LLB/256 nothing (R-MAT scale 19 205 us per BFS instead of 182, 22 to 24 the
+  // same, 25 3.52 ms instead of 3.42) and SLB/256 little (25: 7.7 ms instead of
+  // 8.1), and its build would cost a first call more than many searches: R-MAT
+  // 23, LLB/256, first call 8.7 ms and 1.2 GB with it, 1.1 ms and none without.
+  const bool want_hub = o.lb == BFS_LB_GLB || o.lb == BFS_LB_LEARNED || timer != nullptr;
+  if (want_hub) {
+    const bfs_status hrc = ensure_hub(g);
+    if (hrc != BFS_OK) return hrc;
+  }
   BfsDevState s = g->tmpl;
   s.root = root;
   s.level = levels_dev;
   s.parent = parents_dev;
   s.fixed_arm = arm;
-  // The layout serves plans that run GLB levels (fixed GLB arms, the learned
-  // schedule, the per-level recorder).  Fixed LLB and SLB keep the original
-  // numbering: their tile-local balancing suffers when the hubs are
-  // consecutive ids, i.e. consecutive queue entries.
-  const bool use_hub = g->hub != nullptr &&
-                       (o.lb == BFS_LB_GLB || o.lb == BFS_LB_LEARNED || timer != nullptr);
+  const bool use_hub = want_hub && g->hub != nullptr;
   if (use_hub) {
     s.indptr = g->hub->indptr;
     s.inds = g->hub->inds;

@@ -140,10 +140,10 @@ bfs_status bfs_graph_device_csc(const bfs_graph *g, const uint32_t **d_indptr,
  * whose internal ids 0 .. K-1 are its K highest in-degree vertices (graphs
  * of at most K vertices, and graphs with n_rows < n_cols, keep their own ids
  * and no copy).  The layout serves runs whose plan runs GLB levels (fixed
- * GLB arms and the learned schedule); fixed LLB and SLB runs keep the
- * original numbering, since their tile-local balancing suffers when the hubs
- * are consecutive ids.  Levels, parents and every other entry point still
- * use the caller's ids; results are identical with or without the layout.  The copy
+ * GLB arms and the learned schedule); fixed LLB and SLB runs search the
+ * caller's numbering, which serves them as well.  Levels, parents and every
+ * other entry point still use the caller's ids; results are identical with or
+ * without the layout.  The copy
  * costs nnz + 8 n_cols + 1 uint32 of device memory; if it cannot be
  * allocated the handle runs without it.  The copy's lists are ordered by the
  * targets' degree class; once all vertices of the highest classes are
@@ -154,7 +154,8 @@ bfs_status bfs_graph_device_csc(const bfs_graph *g, const uint32_t **d_indptr,
  * shared memory), 0 = off, > 0 = K (rounded down to a multiple of 128).
  * min_edges: the smallest level (frontier edges) for which the explore
  * kernel loads the prefix into shared memory; 0 = automatic (max(2^21, 2K)).
- * The layout is built by this call, or by the first single-root run. */
+ * The layout is built by this call, by bfs_hub_info, or by the first run that
+ * it serves (single-root GLB, learned or recorder runs, batches). */
 bfs_status bfs_hub_configure(bfs_graph *g, int64_t vertices, uint32_t min_edges);
 /* The current layout: *vertices = K (0: none), *relabelled = 1 if the
  * handle holds a relabelled copy, *max_vertices = the largest K the device
