@@ -283,24 +283,24 @@ __device__ __forceinline__ void explore_local_body(const BfsDevState *__restrict
   const uint32_t *__restrict__ qc = st->qc[cur_q];
   const uint32_t eoff = st->inds_off, EC = st->EC;
   uint32_t per = 0, j = 0, x_end = 0;
-  if (!STRIDED) {
-    const uint64_t p = ((uint64_t)EC + nvb - 1) / nvb;
-    per = (uint32_t)(p > (uint64_t)B ? p : (uint64_t)B);
-  }
-  const uint32_t num_ranges = STRIDED ? num_tiles : (uint32_t)(((uint64_t)EC + per - 1) / per);
+  if (!STRIDED) per = max((EC - 1u) / nvb + 1u, (uint32_t)B);  // F > 0: EC > 0
+  const uint32_t num_ranges = STRIDED ? num_tiles : (EC - 1u) / per + 1u;
 
   // STRIDED: one tile per step; otherwise one range, and in it one tile per
   // inner step
   for (uint32_t tile = vb; tile < num_ranges; tile += nvb) {
     const uint32_t x = tile * per;
     if (!STRIDED) {
-      x_end = (uint32_t)min((uint64_t)EC, (uint64_t)x + per);
-      if (warp == 0) {
-        const uint32_t o = warp_owner_search(qc, F, x, lane);
-        if (lane == 0) s_off[0] = o;
+      x_end = x + min(EC - x, per);
+      j = 0;
+      if (x != 0u) {  // the first range starts at entry 0
+        if (warp == 0) {
+          const uint32_t o = warp_owner_search(qc, F, x, lane);
+          if (lane == 0) s_off[0] = o;
+        }
+        vblock_sync<B>(bar);
+        j = s_off[0];
       }
-      vblock_sync<B>(bar);
-      j = s_off[0];
     }
     do {
       const uint32_t slot = STRIDED ? tile + tid * num_tiles : j + tid;
