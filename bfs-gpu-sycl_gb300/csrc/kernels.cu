@@ -409,8 +409,8 @@ __global__ void __launch_bounds__(B, (MinBlocks<B, U, STRIDED>::value))
 // four edge slots.  Owners are resolved with a warp OR-reduction of the next
 // 32 entry starts plus a popc (O(1) per chunk, instead of the reference's
 // per-edge binary search, :336-346).  The slots outside [b, b + deg) -- only
-// in an entry's first and last chunk -- are masked off, and a chunk that
-// reaches outside inds (the first one when off > 0, the last one when the
+// in an entry's first and last chunk -- hold the root's id, which is visited,
+// and a chunk that reaches outside inds (the first one when off > 0, the last one when the
 // array does not fill it) is read with scalar loads of its valid slots
 // only.  U chunks per lane (4 U edge slots) are loaded per group, and the
 // next group's loads are issued before the current group's probes.

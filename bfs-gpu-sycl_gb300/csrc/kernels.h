@@ -25,9 +25,14 @@ constexpr uint32_t kNarrowBlock = 512;
 // 57 us with 32 to 96, 63 with 128, 76 with 512, 105 with 1024.
 constexpr uint32_t kNarrowHeavy = 64;
 constexpr uint32_t kNarrowHeavyBound = 512;  // the same where only a bound on degrees is known
-// Largest level: 84 K edges (R-MAT scale 12) take 23 us in the two-kernel loop
-// and 14 on the cluster, 379 K (scale 14) take 86 us for the whole BFS there
-// and 101 on the cluster.
+// Largest level.  It costs the cluster by its new vertices, whose entries and
+// levels it writes one by one, more than by its edges.  Whole BFS of a graph
+// with one such level (GLB/256), cluster against two-kernel loop: level of 70 K
+// edges 82 us against 95, 131 K 87 against 98 (103 against 107 with 79 K new
+// vertices), 160 K 90 against 98 (110 against 112 with 96 K new), 200 K 90 to
+// 102 against 97 (138 against 111 with 120 K new), 260 K 166 against 109 with
+// 156 K new.  Above 2^17 a level of few new vertices would still gain a tenth,
+// and nothing tells the two apart beforehand.
 constexpr uint32_t kNarrowEdges = 1u << 17;
 constexpr uint32_t kNarrowList = 8192;         // entries walked by the whole cluster
 constexpr uint32_t kNarrowEntries = 48u << 10;  // they fit the cluster's queues

@@ -569,7 +569,12 @@ __device__ __forceinline__ void ms_expand_rows(const MsState *__restrict__ st, u
   }
 }
 
-// Vertices from which a lane takes four.
+// Vertices from which a lane takes four.  With fewer, the warps that one vertex
+// per lane gives matter more than the runs of a row, with more the runs do:
+// pass of 64 roots, one against four per lane: R-MAT scale 10 176 us against
+// 184, scale 12 188 against 194, ER 5 K vertices 189 against 196; 60 K to 262 K
+// vertices within 1 %; ER 700 K 817 against 792, R-MAT scale 22 2.96 ms against
+// 2.59 (the latter with the other changes to the pass).
 constexpr uint32_t kXvVertices = 1u << 17;
 
 __global__ void __launch_bounds__(kMsBlock, kXb) ms_expand_kernel(MsState *__restrict__ st,
@@ -594,9 +599,6 @@ __global__ void __launch_bounds__(kMsBlock, kXb) ms_expand_kernel(MsState *__res
   const uint64_t gwarp = ((uint64_t)blockIdx.x * kMsBlock + threadIdx.x) >> 5;
   const uint64_t warps = (uint64_t)gridDim.x * (kMsBlock / 32);
   if (expand) {
-    // with few vertices the warps that one vertex per lane gives matter more
-    // than the runs of a row (R-MAT scale 12, 4 roots: 178 us
-    // per call instead of 184)
     if (n >= kXvVertices) ms_expand_rows<4>(st, lmax, gwarp, warps);
     else ms_expand_rows<1>(st, lmax, gwarp, warps);
   }

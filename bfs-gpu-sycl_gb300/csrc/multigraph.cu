@@ -10,8 +10,8 @@
 // as the level barrier.  Within a level the block uses the LLB form: a block
 // exclusive scan of a tile's degrees, the tile's edges split evenly over the
 // warps, owners resolved per warp round (bfs_internal / device_util), a 16-byte
-// chunk of edges or one edge per lane.  A claim is an atomicOr on the shared bitmap; the
-// claiming thread writes the level and appends the vertex to the next queue
+// chunk of edges or one edge per lane.  A claim is an atomicOr on the shared
+// bitmap; the claiming thread writes the level and appends the vertex to the next queue
 // (vertices >= n_rows get a level but are not queued; those without out-edges
 // are dropped when the next level loads their offsets).
 //
@@ -293,8 +293,9 @@ __global__ void __launch_bounds__(B, 2048 / B) multi_bfs_kernel(MultiArgs a) {
 // Clusters of C blocks first share the largest graphs (order[0, n_big)): a
 // claimed graph's frontier tiles are dealt round-robin over the cluster's
 // blocks, claims go to the cluster's bitmap in global memory (L2), every
-// block keeps a shared-memory copy of the visited set as a filter (merged
-// from the new frontier after every level), the level barrier is the
+// block keeps a shared-memory copy of the visited set as a filter (after every
+// level merged from the new frontier, or copied whole where the bitmap is the
+// shorter of the two), the level barrier is the
 // cluster barrier, and the next frontier is one queue per cluster with
 // counters in global memory.  Then every block takes small graphs on its
 // own.  Each frontier entry is expanded by exactly one block, so the edge

@@ -29,7 +29,7 @@
 // Measured per level, learned plan: 2.5 us on a 300 x 300 grid (200 entries a
 // level) against 18.3 in the two-kernel loop, 4.6 against 21.8 on 4096 x 4096
 // (3600 entries, where the scattered loads and claims of 16 SMs bound it);
-// R-MAT scale 12, whole BFS: 63 us against 117.  Blocks of 512 threads: 1024
+// R-MAT scale 12, whole BFS: 57 us against 117.  Blocks of 512 threads: 1024
 // spill and wait longer at the barrier (2.8 -> 4.3 us on 1023 x 1537), 256
 // have too few lanes (4.6 -> 7.3 on 4096 x 4096).  Clusters of 8 instead of
 // 16: 5.6 -> 7.4 there in an earlier form.  With the queue in global memory

@@ -79,8 +79,9 @@ typedef struct bfs_options {
                           runs its arm's explore kernel on its whole frontier);
                           2 = also time every kernel with CUDA events (forces
                           the host loop) */
-  int32_t ipt;         /* edges per lane in flight in the explore kernels:
-                          4 or 8 (0 = 4) */
+  int32_t ipt;         /* edges per lane in flight in the LLB and SLB explore
+                          kernels: 4 or 8 (0 = 4); the GLB walk sets its own
+                          by the size of the level */
 } bfs_options;
 
 #define BFS_MAX_RECORDED_LEVELS 4096
@@ -257,8 +258,9 @@ bfs_status bfs_multi_autotune(bfs_multi *m, const uint32_t *roots, int32_t *leve
                               int32_t reps, const char *cache_path, int32_t *best_block,
                               int32_t *best_ipt, float *times_ms);
 /* bfs_multi_run with cluster > 1: the batch's largest graphs (edge count at
- * least `cluster` blocks' fair share of the batch) are each run by a cluster
- * of `cluster` thread blocks (tiles of the frontier dealt over the cluster,
+ * least `cluster` blocks' fair share of the batch, or a quarter of that share
+ * and 2^17 edges) are each run by a cluster of `cluster` thread blocks (tiles
+ * of the frontier dealt over the cluster,
  * claims on a per-cluster bitmap in L2, the cluster barrier as the level
  * barrier); the other graphs run one per block as above.  Configurations:
  * cluster 1 with block 128/256/512 and ipt 1/2/4; cluster 2/4/8 with block
