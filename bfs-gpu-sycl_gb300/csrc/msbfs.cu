@@ -95,6 +95,7 @@ struct MsState {
   const uint32_t *skip[kHubClasses];
   uint32_t skip_limit[kHubClasses];
   uint32_t skip_classes;
+  uint32_t skip_min_edges;  // frontier edges from which a level looks for more of them
   uint32_t full;      // classes known to be reached by every root
   uint32_t not_full;  // bit c: class c has a vertex some root has not reached
   uint32_t n_lanes;
@@ -268,14 +269,24 @@ __global__ void __launch_bounds__(kMsBlock, 1536 / kMsBlock)
   }
 }
 
-// Classes reached by every root, after ms_between_classes has looked.
-__device__ __forceinline__ uint32_t ms_full_classes(const MsState *st) {
-  const uint32_t nf = st->not_full;
-  const uint32_t first = nf ? (uint32_t)__ffs(nf) - 1u : st->skip_classes;
-  return first < st->skip_classes ? first : st->skip_classes;
+// Whether the level between explore and level generation looks for classes
+// reached by every root.  Levels of few edges don't: what they could leave out
+// of the next one is not worth the look (a round trip per level: ER 700 K
+// vertices, one root, 2.7 us on each of 11 levels).
+__device__ __forceinline__ bool ms_looks(const MsState *st) {
+  return st->skip_classes != 0u && st->EF >= st->skip_min_edges;
 }
 
-__device__ void ms_finish(MsState *st, unsigned long long cond, int use_cond) {
+// Classes reached by every root, after ms_between_classes has looked, if it has.
+__device__ __forceinline__ uint32_t ms_full_classes(const MsState *st) {
+  const uint32_t nf = st->not_full, classes = st->skip_classes, known = st->full;
+  const uint32_t first = nf ? (uint32_t)__ffs(nf) - 1u : classes;
+  return ms_looks(st) ? (first < classes ? first : classes) : known;
+}
+
+// `full`: the classes reached by every root, as the caller has read them (read
+// here, behind the stores, they cost each level another round trip).
+__device__ void ms_finish(MsState *st, uint32_t full, unsigned long long cond, int use_cond) {
   const unsigned long long packed = *(volatile unsigned long long *)&st->next_packed;
   const uint32_t f_new = (uint32_t)(packed >> 32), ef_new = (uint32_t)packed;
   const uint32_t lvl = st->lvl + 1;
@@ -289,7 +300,7 @@ __device__ void ms_finish(MsState *st, unsigned long long cond, int use_cond) {
   st->lvl = lvl;
   st->next_packed = 0;
   st->done_blocks = 0;
-  st->full = ms_full_classes(st);
+  st->full = full;
   st->not_full = 0;
   st->launches += 3;  // explore, classes and expand check, levelgen
   if (f_new > 0 && lvl >= st->level_cap) {
@@ -348,10 +359,10 @@ __global__ void __launch_bounds__(kMsBlock) ms_levelgen_kernel(MsState *__restri
     const uint32_t v = (uint32_t)(sb + threadIdx.x);
     unsigned long long nw = 0;
     uint32_t b = 0, e = 0;
-    bool full = false;
+    bool by_all = false;
     if (v < n_cols) {
       const unsigned long long vv = vis[v];
-      full = vv == all_roots;
+      by_all = vv == all_roots;
       nw = vv & ~prev[v];
       if (nw) {
         prev[v] = vv;
@@ -366,7 +377,7 @@ __global__ void __launch_bounds__(kMsBlock) ms_levelgen_kernel(MsState *__restri
     any |= nw != 0;
     // hub ids every root has reached (warps cover 32 aligned ids)
     if (hub_words) {
-      const uint32_t fm = __ballot_sync(kFull, full);
+      const uint32_t fm = __ballot_sync(kFull, by_all);
       if (lane == 0 && (v >> 5) < hub_words) hubfull[v >> 5] = fm;
     }
     if (!hist) {  // past the history: one root row at a time
@@ -419,7 +430,7 @@ __global__ void __launch_bounds__(kMsBlock) ms_levelgen_kernel(MsState *__restri
   __syncthreads();
   if (s_last && threadIdx.x == 0) {
     __threadfence();
-    ms_finish(st, cond, use_cond);
+    ms_finish(st, full, cond, use_cond);
   }
 }
 
@@ -445,10 +456,10 @@ __device__ __forceinline__ void ms_between_classes(MsState *st) {
   }
 }
 
-// In the level loop (final == 0, between explore and level generation): looks
-// for classes reached by every root and, when the next level is the first past
+// In the level loop (FINAL false, between explore and level generation): looks
+// for classes reached by every root (ms_looks) and, when the next level is the first past
 // the history, writes every row entry (level or -1) so that level generation
-// can write the deeper levels directly.  After the loop (final != 0) it writes
+// can write the deeper levels directly.  After the loop (FINAL) it writes
 // the rows unless that already happened (the search went past the history),
 // then adds, per root, the degrees of the vertices < n_rows it reached
 // (run_bfs_cpu.hpp:36).
@@ -577,15 +588,15 @@ __device__ __forceinline__ void ms_expand_rows(const MsState *__restrict__ st, u
 // 2.59 (the latter with the other changes to the pass).
 constexpr uint32_t kXvVertices = 1u << 17;
 
-__global__ void __launch_bounds__(kMsBlock, kXb) ms_expand_kernel(MsState *__restrict__ st,
-                                                                  int final) {
+template <bool FINAL>
+__global__ void __launch_bounds__(kMsBlock, kXb) ms_expand_kernel(MsState *__restrict__ st) {
   static_assert(kHistLevels <= 16, "levels must fit four bit planes");
   __shared__ unsigned long long s_edges[kLanes];
   __shared__ unsigned long long s_common;
   const uint32_t lvl = st->lvl;
-  const bool expand = final ? (lvl < kHistLevels) : (lvl + 1u == kHistLevels);
-  if (!final) {
-    if (st->skip_classes) ms_between_classes(st);
+  const bool expand = FINAL ? (lvl < kHistLevels) : (lvl + 1u == kHistLevels);
+  if constexpr (!FINAL) {
+    if (ms_looks(st)) ms_between_classes(st);
     if (!expand) return;  // uniform over the grid
   }
   const uint32_t n_rows = st->n_rows, nl = st->n_lanes;
@@ -602,7 +613,7 @@ __global__ void __launch_bounds__(kMsBlock, kXb) ms_expand_kernel(MsState *__res
     if (n >= kXvVertices) ms_expand_rows<4>(st, lmax, gwarp, warps);
     else ms_expand_rows<1>(st, lmax, gwarp, warps);
   }
-  if (!final) return;
+  if constexpr (!FINAL) return;
   if (threadIdx.x < kLanes) s_edges[threadIdx.x] = 0;
   if (threadIdx.x == 0) s_common = 0;
   __syncthreads();
@@ -750,6 +761,7 @@ static bfs_status ms_setup(bfs_graph *g) {
     }
     s.hub_min_edges = g->hub_min_edges ? g->hub_min_edges
                                        : std::max<uint32_t>(kHubMinEdges, 2u * ms_hub);
+    s.skip_min_edges = s.hub_min_edges >> 4;  // as in single-root runs
     if (hub_bytes > 48 * 1024)
       MK(cudaFuncSetAttribute((const void *)ms_explore_kernel,
                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hub_bytes));
@@ -769,7 +781,7 @@ static bfs_status ms_setup(bfs_graph *g) {
                                                    kMsBlock, hub_bytes));
   MK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_lg, (const void *)ms_levelgen_kernel,
                                                    kMsBlock, 0));
-  MK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_xp, (const void *)ms_expand_kernel,
+  MK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_xp, (const void *)ms_expand_kernel<true>,
                                                    kMsBlock, 0));
   w->grid_ex = g->num_sms * std::max(occ_ex, 1);
   w->grid_lg = g->num_sms * std::max(occ_lg, 1);
@@ -825,9 +837,8 @@ static bfs_status ms_setup(bfs_graph *g) {
   kp.kernelParams = ex_args;
   MK(cudaGraphAddKernelNode(&n_ex, body, nullptr, 0, &kp));
   kp.sharedMemBytes = 0;
-  int in_loop = 0, after = 1;
-  void *xp_args[] = {&st, &in_loop};
-  kp.func = (void *)ms_expand_kernel;
+  void *xp_args[] = {&st};
+  kp.func = (void *)ms_expand_kernel<false>;
   kp.gridDim = dim3(w->grid_xp);
   kp.blockDim = dim3(kMsBlock);
   kp.kernelParams = xp_args;
@@ -837,10 +848,9 @@ static bfs_status ms_setup(bfs_graph *g) {
   kp.gridDim = dim3(w->grid_lg);
   kp.kernelParams = lg_args;
   MK(cudaGraphAddKernelNode(&n_lg, body, &n_xp, 1, &kp));
-  kp.func = (void *)ms_expand_kernel;
+  kp.func = (void *)ms_expand_kernel<true>;
   kp.gridDim = dim3(w->grid_xp);
-  void *xf_args[] = {&st, &after};
-  kp.kernelParams = xf_args;
+  kp.kernelParams = xp_args;
   MK(cudaGraphAddKernelNode(&n_xf, w->graph, &n_while, 1, &kp));
   MK(cudaGraphInstantiate(&w->exec, w->graph, 0));
   return BFS_OK;
@@ -865,12 +875,12 @@ static bfs_status ms_pass_host(bfs_graph *g, MsWorkspace *w) {
     if (*h_F == 0) break;
     ms_explore_kernel<<<w->grid_ex, kMsBlock, w->hub_bytes, s>>>(st);
     MK(cudaGetLastError());
-    ms_expand_kernel<<<w->grid_xp, kMsBlock, 0, s>>>(st, 0);
+    ms_expand_kernel<false><<<w->grid_xp, kMsBlock, 0, s>>>(st);
     MK(cudaGetLastError());
     ms_levelgen_kernel<<<w->grid_lg, kMsBlock, 0, s>>>(st, no_cond, zero);
     MK(cudaGetLastError());
   }
-  ms_expand_kernel<<<w->grid_xp, kMsBlock, 0, s>>>(st, 1);
+  ms_expand_kernel<true><<<w->grid_xp, kMsBlock, 0, s>>>(st);
   MK(cudaGetLastError());
   return BFS_OK;
 }
