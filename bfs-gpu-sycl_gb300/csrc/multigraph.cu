@@ -11,9 +11,10 @@
 // exclusive scan of a tile's degrees, the tile's edges split evenly over the
 // warps, owners resolved per warp round (bfs_internal / device_util), a 16-byte
 // chunk of edges or one edge per lane.  A claim is an atomicOr on the shared
-// bitmap; the claiming thread writes the level and appends the vertex to the next queue
-// (vertices >= n_rows get a level but are not queued; those without out-edges
-// are dropped when the next level loads their offsets).
+// bitmap; the claiming thread writes the level and appends the vertex to the
+// next queue (vertices >= n_rows get a level but are not queued; those without
+// out-edges are not queued either in batches with many of them, and otherwise
+// dropped when the next level loads their offsets).
 //
 // Block size (128/256/512), the form of a round (items per thread: 1 for single
 // edges, 2 or 4 for chunks) and the cluster size come from an autotuner that
@@ -39,12 +40,23 @@
 namespace bfsgb {
 
 constexpr uint32_t kShareEdges = 1u << 17;
+// Share of the batch's edges (1 in kLeafShare) that point at vertices without
+// out-edges from which those are not queued.  Queueing them costs a pass over
+// their offsets, keeping them out a load beside every claim.  Random directed
+// graphs, a share f of the vertices without out-edges, 512 threads and chunks,
+// queued against kept out, us: 12 of 200 K vertices 2109 / 2258 (f = 0.01), 2099
+// / 2071 (0.1), 2072 / 1861 (0.2), 1701 / 1626 (0.3), 952 / 644 (0.7); 32 of
+// 40 K 393 / 418, 396 / 393, 415 / 379, 345 / 325, 246 / 184; 64 of 3 K vertices
+// within noise at every f; single edges cross at 0.3.  Symmetric graphs have no
+// such edge.
+constexpr uint64_t kLeafShare = 4;
 constexpr uint32_t kMultiMaxVertices = 1u << 18;  // 32 KiB shared bitmap
 
 struct MultiDesc {
   uint64_t vbase;      // offset of the graph's indptr in the packed indptr array
   uint64_t ebase;      // offset of the graph's edges in the packed inds array
   uint64_t lbase;      // offset of the graph's levels in the output
+  uint64_t wbase;      // offset of its words in the expandable-vertex bitmaps
   uint32_t n_rows, n_cols;
   uint32_t root;
   uint32_t pad;
@@ -58,6 +70,7 @@ struct MultiArgs {
   uint32_t n_big;               // order[0, n_big): graphs run by a whole cluster
   const uint32_t *indptr_all;
   const uint32_t *inds_all;
+  const uint32_t *expandable;   // per graph: bit v: v < n_rows and v has out-edges
   uint32_t *work;               // [0]: next small graph, [1]: next big graph
   uint32_t *queues;             // two queues of qcap entries per block
   uint32_t qcap;
@@ -90,7 +103,9 @@ struct MultiTile {
 // filter of already visited vertices; a lane's claims are in flight together.
 // The claiming thread writes the level; the warp's new vertices are appended to
 // qn through one atomic on *ctr (shared, or global for CL).  Their degrees are
-// not looked at here, so no dependent load waits in the innermost loop.
+// not looked at here, so no dependent load waits in the innermost loop; LEAVES
+// loads each target's bit of the expandable vertices (ob) beside its claim
+// instead and appends only those (kLeafShare has both sides).
 // Returns this thread's part of the sum of the tiles' degrees.  Bound by
 // instruction issue on the busiest SMs; 256 R-MAT graphs of scales 10-16, best
 // configuration 1.10 -> 0.59 ms: without the degree look-up and one-by-one
@@ -99,12 +114,12 @@ struct MultiTile {
 // instead of a whole one as the limit for sharing a graph 0.93 -> 0.78 (half,
 // eighth, sixteenth: 0.79, 0.78, 0.81); chunks 0.78 -> 0.59.  Registers for 2
 // or 3 blocks of 512 threads per SM instead of 4: 0.80, 0.76.
-template <int B, bool CHUNKS, bool CL>
+template <int B, bool CHUNKS, bool CL, bool LEAVES>
 __device__ __forceinline__ unsigned long long multi_level(
     const uint32_t *__restrict__ ip, const uint32_t *__restrict__ ix, int32_t *lv,
-    uint32_t n_rows, const uint32_t *qc, uint32_t *qn, uint32_t F, int32_t lvl,
-    uint32_t tile0, uint32_t tstride, uint32_t *s_bitmap, uint32_t *gb, uint32_t *ctr,
-    MultiTile<B> &s) {
+    uint32_t n_rows, const uint32_t *__restrict__ ob, const uint32_t *qc, uint32_t *qn,
+    uint32_t F, int32_t lvl, uint32_t tile0, uint32_t tstride, uint32_t *s_bitmap, uint32_t *gb,
+    uint32_t *ctr, MultiTile<B> &s) {
   constexpr int NW = B / 32;
   constexpr int kSlots = CHUNKS ? 4 : 1;  // edges per lane
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -185,13 +200,14 @@ __device__ __forceinline__ unsigned long long multi_level(
           on = e < w1 ? 1u : 0u;
           nb[0] = e < w1 ? ix[s.beg[o] + (e - s.off[o])] : 0u;
         }
-        uint32_t old[kSlots];
+        uint32_t old[kSlots], can[LEAVES ? kSlots : 1];
 #pragma unroll
         for (int u = 0; u < kSlots; u++) {
           const uint32_t w = nb[u] >> 5, bit = 1u << (nb[u] & 31u);
           old[u] = kFull;  // visited
           if (((on >> u) & 1u) && !(s_bitmap[w] & bit)) {
             old[u] = atomicOr((CL ? gb : s_bitmap) + w, bit);
+            if (LEAVES) can[u] = __ldg(ob + w);
             if (CL) atomicOr(s_bitmap + w, bit);
           }
         }
@@ -200,7 +216,10 @@ __device__ __forceinline__ unsigned long long multi_level(
         for (int u = 0; u < kSlots; u++) {
           const bool mine = !((old[u] >> (nb[u] & 31u)) & 1u);
           if (mine) lv[nb[u]] = lvl + 1;
-          push[u] = __ballot_sync(kFull, mine && nb[u] < n_rows);
+          // one expression: with its second half in a variable of its own the
+          // compiler's code for clusters is a fifth slower (0.64 -> 0.78 ms)
+          push[u] = __ballot_sync(
+              kFull, mine && (LEAVES ? (bool)((can[u] >> (nb[u] & 31u)) & 1u) : nb[u] < n_rows));
           num += __popc(push[u]);
         }
         if (num == 0u) continue;  // uniform over the warp
@@ -228,12 +247,13 @@ __device__ __forceinline__ void add_edges(unsigned long long *out, unsigned long
 
 // A complete BFS of one graph by one block, the visited bitmap in shared
 // memory and __syncthreads as the level barrier.
-template <int B, bool CHUNKS>
+template <int B, bool CHUNKS, bool LEAVES>
 __device__ __forceinline__ void multi_graph_block(const MultiArgs &a, uint32_t gi,
                                                   uint32_t *s_bitmap, MultiTile<B> &s) {
   const MultiDesc d = a.descs[a.order[gi]];
   const uint32_t *__restrict__ ip = a.indptr_all + d.vbase;
   const uint32_t *__restrict__ ix = a.inds_all + d.ebase;
+  const uint32_t *ob = LEAVES ? a.expandable + d.wbase : nullptr;
   int32_t *lv = a.levels + d.lbase;
   uint32_t *q0 = a.queues + (size_t)blockIdx.x * 2 * a.qcap;
   uint32_t *q1 = q0 + a.qcap;
@@ -257,8 +277,8 @@ __device__ __forceinline__ void multi_graph_block(const MultiArgs &a, uint32_t g
     __syncthreads();
     if (threadIdx.x == 0) s.next = 0;
     __syncthreads();
-    edges += multi_level<B, CHUNKS, false>(ip, ix, lv, d.n_rows, qc, qn, F, lvl, 0u, B, s_bitmap,
-                                        nullptr, &s.next, s);
+    edges += multi_level<B, CHUNKS, false, LEAVES>(ip, ix, lv, d.n_rows, ob, qc, qn, F, lvl, 0u, B,
+                                                   s_bitmap, nullptr, &s.next, s);
     __syncthreads();
     F = s.next;
     uint32_t *t = qc;
@@ -270,7 +290,7 @@ __device__ __forceinline__ void multi_graph_block(const MultiArgs &a, uint32_t g
 }
 
 // Graphs claimed one per block from a work counter (largest first).
-template <int B, bool CHUNKS>
+template <int B, bool CHUNKS, bool LEAVES>
 __device__ __forceinline__ void multi_small_graphs(const MultiArgs &a, uint32_t *s_bitmap,
                                                    MultiTile<B> &s) {
   for (;;) {
@@ -278,16 +298,16 @@ __device__ __forceinline__ void multi_small_graphs(const MultiArgs &a, uint32_t 
     __syncthreads();
     const uint32_t gi = s.graph;
     if (gi >= a.n_graphs) break;
-    multi_graph_block<B, CHUNKS>(a, gi, s_bitmap, s);
+    multi_graph_block<B, CHUNKS, LEAVES>(a, gi, s_bitmap, s);
     __syncthreads();
   }
 }
 
-template <int B, bool CHUNKS>
+template <int B, bool CHUNKS, bool LEAVES>
 __global__ void __launch_bounds__(B, 2048 / B) multi_bfs_kernel(MultiArgs a) {
   extern __shared__ uint32_t s_bitmap[];
   __shared__ MultiTile<B> s;
-  multi_small_graphs<B, CHUNKS>(a, s_bitmap, s);
+  multi_small_graphs<B, CHUNKS, LEAVES>(a, s_bitmap, s);
 }
 
 // Clusters of C blocks first share the largest graphs (order[0, n_big)): a
@@ -300,7 +320,7 @@ __global__ void __launch_bounds__(B, 2048 / B) multi_bfs_kernel(MultiArgs a) {
 // counters in global memory.  Then every block takes small graphs on its
 // own.  Each frontier entry is expanded by exactly one block, so the edge
 // counts stay exact.
-template <int B, int C>
+template <int B, int C, bool LEAVES>
 __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(B, 2048 / B)
     multi_bfs_cluster_kernel(MultiArgs a) {
   extern __shared__ uint32_t s_bitmap[];
@@ -324,6 +344,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(B, 2048 / B)
     const MultiDesc d = a.descs[a.order[gi]];
     const uint32_t *__restrict__ ip = a.indptr_all + d.vbase;
     const uint32_t *__restrict__ ix = a.inds_all + d.ebase;
+    const uint32_t *ob = LEAVES ? a.expandable + d.wbase : nullptr;
     int32_t *lv = a.levels + d.lbase;
     const uint32_t words = (d.n_cols + 31u) >> 5;
     for (uint32_t w = rank * B + threadIdx.x; w < words; w += C * B) gb[w] = 0u;
@@ -349,8 +370,8 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(B, 2048 / B)
       uint32_t *qc = (lvl & 1) ? cq1 : cq0;
       uint32_t *qn = (lvl & 1) ? cq0 : cq1;
       uint32_t *ctr = cnt + (lvl + 1) % 3;
-      edges += multi_level<B, true, true>(ip, ix, lv, d.n_rows, qc, qn, F, lvl, rank * B, C * B,
-                                         s_bitmap, gb, ctr, s);
+      edges += multi_level<B, true, true, LEAVES>(ip, ix, lv, d.n_rows, ob, qc, qn, F, lvl,
+                                                  rank * B, C * B, s_bitmap, gb, ctr, s);
       cl.sync();
       const uint32_t fn = __ldcg(ctr);
       // vertices claimed by the other blocks join this block's filter: the
@@ -371,7 +392,7 @@ __global__ void __cluster_dims__(C, 1, 1) __launch_bounds__(B, 2048 / B)
     add_edges(a.edges_out + a.order[gi], edges);
     cl.sync();  // queues, counters and bitmap are free for the cluster's next graph
   }
-  multi_small_graphs<B, true>(a, s_bitmap, s);
+  multi_small_graphs<B, true, LEAVES>(a, s_bitmap, s);
 }
 
 __global__ void multi_fill_kernel(int32_t *levels, uint64_t n) {
@@ -380,27 +401,68 @@ __global__ void multi_fill_kernel(int32_t *levels, uint64_t n) {
     levels[i] = -1;
 }
 
+// The bitmaps of expandable vertices: one block per graph.
+__global__ void __launch_bounds__(256) multi_expandable_kernel(
+    const MultiDesc *__restrict__ descs, const uint32_t *__restrict__ indptr_all, uint32_t *bits) {
+  const MultiDesc d = descs[blockIdx.x];
+  const uint32_t *__restrict__ ip = indptr_all + d.vbase;
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t v0 = threadIdx.x & ~31u; v0 < d.n_cols; v0 += 256u) {
+    const uint32_t v = v0 + lane;
+    const uint32_t b = __ballot_sync(kFull, v < d.n_rows && ip[v + 1] > ip[v]);
+    if (lane == 0) bits[d.wbase + (v0 >> 5)] = b;
+  }
+}
+
+// Counts the edges that point at a vertex that is not expandable; gridDim.y
+// blocks per graph.
+__global__ void __launch_bounds__(256) multi_leaves_kernel(
+    const MultiDesc *__restrict__ descs, const uint32_t *__restrict__ indptr_all,
+    const uint32_t *__restrict__ inds_all, const uint32_t *__restrict__ bits,
+    unsigned long long *edges) {
+  const MultiDesc d = descs[blockIdx.x];
+  const uint32_t nnz = indptr_all[d.vbase + d.n_cols];
+  const uint32_t *__restrict__ ix = inds_all + d.ebase;
+  uint32_t n = 0;
+#pragma unroll 4
+  for (uint64_t k = (uint64_t)blockIdx.y * 256u + threadIdx.x; k < nnz; k += gridDim.y * 256u) {
+    const uint32_t v = ix[k];
+    n += !((bits[d.wbase + (v >> 5)] >> (v & 31u)) & 1u);
+  }
+  n = __reduce_add_sync(kFull, n);
+  if ((threadIdx.x & 31u) == 0 && n) atomicAdd(edges, (unsigned long long)n);
+}
+
 using MultiKernel = void (*)(MultiArgs);
 
 struct MultiConfig {
   int block, ipt, cluster;
-  MultiKernel fn;
+  MultiKernel fn[2];  // [1]: LEAVES
 };
 
 // ipt 2 and 4 both name the chunk form.
 static const MultiConfig kMultiConfigs[] = {
-    {128, 1, 1, multi_bfs_kernel<128, false>}, {128, 2, 1, multi_bfs_kernel<128, true>},
-    {128, 4, 1, multi_bfs_kernel<128, true>},
-    {256, 1, 1, multi_bfs_kernel<256, false>}, {256, 2, 1, multi_bfs_kernel<256, true>},
-    {256, 4, 1, multi_bfs_kernel<256, true>},
-    {512, 1, 1, multi_bfs_kernel<512, false>}, {512, 2, 1, multi_bfs_kernel<512, true>},
-    {512, 4, 1, multi_bfs_kernel<512, true>},
-    {256, 2, 2, multi_bfs_cluster_kernel<256, 2>}, {256, 4, 2, multi_bfs_cluster_kernel<256, 2>},
-    {512, 2, 2, multi_bfs_cluster_kernel<512, 2>}, {512, 4, 2, multi_bfs_cluster_kernel<512, 2>},
-    {256, 2, 4, multi_bfs_cluster_kernel<256, 4>}, {256, 4, 4, multi_bfs_cluster_kernel<256, 4>},
-    {512, 2, 4, multi_bfs_cluster_kernel<512, 4>}, {512, 4, 4, multi_bfs_cluster_kernel<512, 4>},
-    {256, 2, 8, multi_bfs_cluster_kernel<256, 8>}, {256, 4, 8, multi_bfs_cluster_kernel<256, 8>},
-    {512, 2, 8, multi_bfs_cluster_kernel<512, 8>}, {512, 4, 8, multi_bfs_cluster_kernel<512, 8>},
+    {128, 1, 1, {multi_bfs_kernel<128, false, false>, multi_bfs_kernel<128, false, true>}},
+    {128, 2, 1, {multi_bfs_kernel<128, true, false>, multi_bfs_kernel<128, true, true>}},
+    {128, 4, 1, {multi_bfs_kernel<128, true, false>, multi_bfs_kernel<128, true, true>}},
+    {256, 1, 1, {multi_bfs_kernel<256, false, false>, multi_bfs_kernel<256, false, true>}},
+    {256, 2, 1, {multi_bfs_kernel<256, true, false>, multi_bfs_kernel<256, true, true>}},
+    {256, 4, 1, {multi_bfs_kernel<256, true, false>, multi_bfs_kernel<256, true, true>}},
+    {512, 1, 1, {multi_bfs_kernel<512, false, false>, multi_bfs_kernel<512, false, true>}},
+    {512, 2, 1, {multi_bfs_kernel<512, true, false>, multi_bfs_kernel<512, true, true>}},
+    {512, 4, 1, {multi_bfs_kernel<512, true, false>, multi_bfs_kernel<512, true, true>}},
+    {256, 2, 2, {multi_bfs_cluster_kernel<256, 2, false>, multi_bfs_cluster_kernel<256, 2, true>}},
+    {256, 4, 2, {multi_bfs_cluster_kernel<256, 2, false>, multi_bfs_cluster_kernel<256, 2, true>}},
+    {512, 2, 2, {multi_bfs_cluster_kernel<512, 2, false>, multi_bfs_cluster_kernel<512, 2, true>}},
+    {512, 4, 2, {multi_bfs_cluster_kernel<512, 2, false>, multi_bfs_cluster_kernel<512, 2, true>}},
+    {256, 2, 4, {multi_bfs_cluster_kernel<256, 4, false>, multi_bfs_cluster_kernel<256, 4, true>}},
+    {256, 4, 4, {multi_bfs_cluster_kernel<256, 4, false>, multi_bfs_cluster_kernel<256, 4, true>}},
+    {512, 2, 4, {multi_bfs_cluster_kernel<512, 4, false>, multi_bfs_cluster_kernel<512, 4, true>}},
+    {512, 4, 4, {multi_bfs_cluster_kernel<512, 4, false>, multi_bfs_cluster_kernel<512, 4, true>}},
+    {256, 2, 8, {multi_bfs_cluster_kernel<256, 8, false>, multi_bfs_cluster_kernel<256, 8, true>}},
+    {256, 4, 8, {multi_bfs_cluster_kernel<256, 8, false>, multi_bfs_cluster_kernel<256, 8, true>}},
+    {512, 2, 8, {multi_bfs_cluster_kernel<512, 8, false>, multi_bfs_cluster_kernel<512, 8, true>}},
+    {512, 4, 8, {multi_bfs_cluster_kernel<512, 8, false>, multi_bfs_cluster_kernel<512, 8, true>}},
 };
 constexpr int kNumMultiConfigs = sizeof(kMultiConfigs) / sizeof(kMultiConfigs[0]);
 constexpr int kNumSingleConfigs = 9;  // the first 9: one block per graph
@@ -424,6 +486,8 @@ struct bfs_multi {
   uint64_t sizes_hash = 0;                           // of all graphs' sizes, in claim order
   uint32_t n_big = 0;
   MultiDesc *d_descs = nullptr;
+  uint32_t *d_expandable = nullptr;  // kept for batches with LEAVES
+  int leaves = 0;  // 1: many edges point at vertices without out-edges (kLeafShare)
   unsigned long long *d_edges = nullptr;
   size_t queue_blocks = 0;
   cudaStream_t stream = nullptr;
@@ -461,10 +525,11 @@ static bfs_status multi_prepare(bfs_multi *m, int cfg, int32_t *levels_dev) {
   const MultiConfig &c = kMultiConfigs[cfg];
   const uint32_t words = (m->max_cols + 31) / 32;
   const size_t smem = (size_t)words * 4;
-  GK(cudaFuncSetAttribute((const void *)c.fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const MultiKernel fn = c.fn[m->leaves];
+  GK(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)std::max<size_t>(smem, 1)));
   int occ = 0;
-  GK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void *)c.fn, c.block, smem));
+  GK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void *)fn, c.block, smem));
   int grid = m->num_sms * std::max(occ, 1);
   grid = (int)std::min<size_t>((size_t)grid, m->queue_blocks);
   uint32_t n_big = 0;
@@ -505,6 +570,7 @@ static bfs_status multi_prepare(bfs_multi *m, int cfg, int32_t *levels_dev) {
   a.n_big = n_big;
   a.indptr_all = m->d_indptr;
   a.inds_all = m->d_inds;
+  a.expandable = m->d_expandable;
   a.work = m->d_work;
   a.queues = m->d_queues;
   a.qcap = m->max_rows;
@@ -519,7 +585,7 @@ static bfs_status multi_prepare(bfs_multi *m, int cfg, int32_t *levels_dev) {
   cudaMemsetAsync(m->d_work, 0, 2 * sizeof(uint32_t), m->stream);
   cudaMemsetAsync(m->d_edges, 0, sizeof(unsigned long long) * m->n_graphs, m->stream);
   multi_fill_kernel<<<m->num_sms * 4, 256, 0, m->stream>>>(levels_dev, m->total_cols);
-  c.fn<<<grid, c.block, smem, m->stream>>>(a);
+  fn<<<grid, c.block, smem, m->stream>>>(a);
   cudaError_t ce = cudaStreamEndCapture(m->stream, &m->graph);
   if (ce != cudaSuccess)
     return fail(BFS_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(ce));
@@ -545,7 +611,7 @@ bfs_status bfs_multi_create(uint32_t n_graphs, const uint32_t *const *indptrs,
   bfs_multi *m = new bfs_multi();
   m->n_graphs = n_graphs;
   m->descs.resize(n_graphs);
-  uint64_t vb = 0, eb = 0, lb = 0;
+  uint64_t vb = 0, eb = 0, lb = 0, wb = 0;
   for (uint32_t g = 0; g < n_graphs; g++) {
     if (!indptrs[g] || (!inds[g] && nnz[g]) || n_cols[g] == 0 || n_rows[g] > n_cols[g] ||
         n_cols[g] > kMultiMaxVertices || nnz[g] > BFS_MAX_EDGES || indptrs[g][n_cols[g]] != nnz[g]) {
@@ -557,12 +623,14 @@ bfs_status bfs_multi_create(uint32_t n_graphs, const uint32_t *const *indptrs,
     d.vbase = vb;
     d.ebase = eb;
     d.lbase = lb;
+    d.wbase = wb;
     d.n_rows = n_rows[g];
     d.n_cols = n_cols[g];
     d.root = 0;
     vb += (uint64_t)n_cols[g] + 1;
     eb += nnz[g];
     lb += n_cols[g];
+    wb += (n_cols[g] + 31u) / 32u;
     m->max_cols = std::max(m->max_cols, n_cols[g]);
     m->max_rows = std::max(m->max_rows, std::max<uint32_t>(n_rows[g], 1));
   }
@@ -607,6 +675,7 @@ bfs_status bfs_multi_create(uint32_t n_graphs, const uint32_t *const *indptrs,
     cudaFree(m->d_work);
     cudaFree(m->d_queues);
     cudaFree(m->d_descs);
+    cudaFree(m->d_expandable);
     cudaFree(m->d_edges);
     if (m->stream) cudaStreamDestroy(m->stream);
     if (m->e0) cudaEventDestroy(m->e0);
@@ -643,6 +712,29 @@ bfs_status bfs_multi_create(uint32_t n_graphs, const uint32_t *const *indptrs,
   CK2(cudaMemcpy(m->d_inds, hix.data(), sizeof(uint32_t) * std::max<uint64_t>(eb, 1),
                  cudaMemcpyHostToDevice));
   CK2(cudaMemcpy(m->d_order, order.data(), sizeof(uint32_t) * n_graphs, cudaMemcpyHostToDevice));
+  // which vertices are expandable, and how many edges point at others (counted
+  // in the first edge count, which is cleared before every launch)
+  {
+    unsigned long long to_leaves = 0;
+    CK2(dev_malloc(&m->d_expandable, sizeof(uint32_t) * wb));
+    CK2(cudaMemcpyAsync(m->d_descs, m->descs.data(), sizeof(MultiDesc) * n_graphs,
+                        cudaMemcpyHostToDevice, m->stream));
+    CK2(cudaMemsetAsync(m->d_edges, 0, sizeof(to_leaves), m->stream));
+    multi_expandable_kernel<<<n_graphs, 256, 0, m->stream>>>(m->d_descs, m->d_indptr,
+                                                             m->d_expandable);
+    const uint32_t slices = (uint32_t)std::min<uint64_t>(64, eb / n_graphs / 4096 + 1);
+    multi_leaves_kernel<<<dim3(n_graphs, slices), 256, 0, m->stream>>>(
+        m->d_descs, m->d_indptr, m->d_inds, m->d_expandable, m->d_edges);
+    CK2(cudaGetLastError());
+    CK2(cudaMemcpyAsync(&to_leaves, m->d_edges, sizeof(to_leaves), cudaMemcpyDeviceToHost,
+                        m->stream));
+    CK2(cudaStreamSynchronize(m->stream));
+    m->leaves = to_leaves * kLeafShare >= eb && to_leaves > 0 ? 1 : 0;
+    if (!m->leaves) {
+      CK2(cudaFree(m->d_expandable));
+      m->d_expandable = nullptr;
+    }
+  }
 #undef CK2
   *out = m;
   return BFS_OK;
@@ -662,6 +754,7 @@ bfs_status bfs_multi_free(bfs_multi *m) {
   cudaFree(m->d_gbits);
   cudaFree(m->d_gcnt);
   cudaFree(m->d_descs);
+  cudaFree(m->d_expandable);
   cudaFree(m->d_edges);
   if (m->stream) cudaStreamDestroy(m->stream);
   if (m->e0) cudaEventDestroy(m->e0);
@@ -720,12 +813,12 @@ bfs_status bfs_multi_run_ex(bfs_multi *m, const uint32_t *roots, int32_t block, 
 
 // Raised whenever a kernel or the rule for sharing graphs changes: a choice
 // cached before was timed on other code.
-constexpr int kMultiRevision = 3;
+constexpr int kMultiRevision = 4;
 
 // Times the kernels of configurations [0, n_cfg) on the batch (best of reps after a warm-up
 // run that also captures the launch) and returns the fastest; a cache file
-// keeps the choice per GPU, kernel revision, configuration set and sizes of the
-// batch's graphs (batches of equal totals differ in what clusters share).
+// keeps the choice per GPU, kernel revision and form, configuration set and sizes
+// of the batch's graphs (batches of equal totals differ in what clusters share).
 static bfs_status multi_autotune(bfs_multi *m, const uint32_t *roots, int32_t *levels_dev,
                                  int32_t reps, const char *cache_path, int n_cfg, int *best_out,
                                  float *times_ms) {
@@ -736,7 +829,7 @@ static bfs_status multi_autotune(bfs_multi *m, const uint32_t *roots, int32_t *l
   std::ostringstream key;
   key << prop.name << "|sm" << prop.multiProcessorCount << "|g" << m->n_graphs << "|v"
       << m->total_cols << "|e" << m->total_edges << "|c" << n_cfg << "|h" << std::hex
-      << m->sizes_hash << "|r" << std::dec << kMultiRevision;
+      << m->sizes_hash << "|l" << m->leaves << "|r" << std::dec << kMultiRevision;
   if (cache_path && cache_path[0]) {
     std::ifstream in(cache_path);
     std::string line;
@@ -760,7 +853,7 @@ static bfs_status multi_autotune(bfs_multi *m, const uint32_t *roots, int32_t *l
   for (int i = 0; i < n_cfg; i++) {
     const MultiConfig &c = kMultiConfigs[i];
     int same = 0;  // a configuration before it with the same kernel is not timed again
-    while (kMultiConfigs[same].fn != c.fn) same++;
+    while (kMultiConfigs[same].fn[0] != c.fn[0]) same++;
     if (same < i) {
       if (times_ms) times_ms[i] = times_ms[same];
       continue;
