@@ -401,9 +401,12 @@ __global__ void multi_fill_kernel(int32_t *levels, uint64_t n) {
     levels[i] = -1;
 }
 
-// The bitmaps of expandable vertices: one block per graph.
+// The bitmaps of expandable vertices: one block per graph.  Clears the count of
+// the kernel below.
 __global__ void __launch_bounds__(256) multi_expandable_kernel(
-    const MultiDesc *__restrict__ descs, const uint32_t *__restrict__ indptr_all, uint32_t *bits) {
+    const MultiDesc *__restrict__ descs, const uint32_t *__restrict__ indptr_all, uint32_t *bits,
+    unsigned long long *edges) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *edges = 0ull;
   const MultiDesc d = descs[blockIdx.x];
   const uint32_t *__restrict__ ip = indptr_all + d.vbase;
   const uint32_t lane = threadIdx.x & 31u;
@@ -656,11 +659,15 @@ bfs_status bfs_multi_create(uint32_t n_graphs, const uint32_t *const *indptrs,
     if (nnz[g]) std::memcpy(hix.data() + m->descs[g].ebase, inds[g], sizeof(uint32_t) * nnz[g]);
   }
   unsigned long long bad = 0;
+  bool all_expandable = true;
   for (uint32_t g = 0; g < n_graphs && !bad; g++) {
     const uint32_t *ip = indptrs[g];
     if (ip[0] != 0) bad = 1;
-    for (uint32_t v = 0; v < n_cols[g] && !bad; v++)
+    all_expandable &= n_rows[g] == n_cols[g];
+    for (uint32_t v = 0; v < n_cols[g] && !bad; v++) {
       if (ip[v + 1] < ip[v]) bad = 1;
+      all_expandable &= ip[v + 1] != ip[v];
+    }
     for (uint64_t k = 0; k < nnz[g] && !bad; k++)
       if (inds[g][k] >= n_cols[g]) bad = 1;
   }
@@ -712,27 +719,31 @@ bfs_status bfs_multi_create(uint32_t n_graphs, const uint32_t *const *indptrs,
   CK2(cudaMemcpy(m->d_inds, hix.data(), sizeof(uint32_t) * std::max<uint64_t>(eb, 1),
                  cudaMemcpyHostToDevice));
   CK2(cudaMemcpy(m->d_order, order.data(), sizeof(uint32_t) * n_graphs, cudaMemcpyHostToDevice));
-  // which vertices are expandable, and how many edges point at others (counted
-  // in the first edge count, which is cleared before every launch)
-  {
+  // Which vertices are expandable, and how many edges point at others: counted in
+  // the first edge count, which is cleared before every launch, on a bitmap that
+  // lies in the queues' memory (an allocation of its own, freed again, made a
+  // small batch's creation a tenth longer) unless it has to be kept.
+  if (!all_expandable) {
+    const bool fits = wb <= 2ull * m->max_rows * m->queue_blocks;
     unsigned long long to_leaves = 0;
-    CK2(dev_malloc(&m->d_expandable, sizeof(uint32_t) * wb));
+    if (!fits) CK2(dev_malloc(&m->d_expandable, sizeof(uint32_t) * wb));
+    uint32_t *bits = fits ? m->d_queues : m->d_expandable;
     CK2(cudaMemcpyAsync(m->d_descs, m->descs.data(), sizeof(MultiDesc) * n_graphs,
                         cudaMemcpyHostToDevice, m->stream));
-    CK2(cudaMemsetAsync(m->d_edges, 0, sizeof(to_leaves), m->stream));
-    multi_expandable_kernel<<<n_graphs, 256, 0, m->stream>>>(m->d_descs, m->d_indptr,
-                                                             m->d_expandable);
+    multi_expandable_kernel<<<n_graphs, 256, 0, m->stream>>>(m->d_descs, m->d_indptr, bits,
+                                                             m->d_edges);
     const uint32_t slices = (uint32_t)std::min<uint64_t>(64, eb / n_graphs / 4096 + 1);
     multi_leaves_kernel<<<dim3(n_graphs, slices), 256, 0, m->stream>>>(
-        m->d_descs, m->d_indptr, m->d_inds, m->d_expandable, m->d_edges);
+        m->d_descs, m->d_indptr, m->d_inds, bits, m->d_edges);
     CK2(cudaGetLastError());
     CK2(cudaMemcpyAsync(&to_leaves, m->d_edges, sizeof(to_leaves), cudaMemcpyDeviceToHost,
                         m->stream));
     CK2(cudaStreamSynchronize(m->stream));
     m->leaves = to_leaves * kLeafShare >= eb && to_leaves > 0 ? 1 : 0;
-    if (!m->leaves) {
-      CK2(cudaFree(m->d_expandable));
-      m->d_expandable = nullptr;
+    if (m->leaves && fits) {
+      CK2(dev_malloc(&m->d_expandable, sizeof(uint32_t) * wb));
+      CK2(cudaMemcpyAsync(m->d_expandable, bits, sizeof(uint32_t) * wb, cudaMemcpyDeviceToDevice,
+                          m->stream));
     }
   }
 #undef CK2

@@ -71,3 +71,25 @@ def test_batch_without_edges(B):
     want[0] = want[1 + 7] = 0
     assert np.array_equal(out.cpu().numpy(), want) and list(ec) == [0, 0]
     batch.free()
+
+
+def test_bitmap_larger_than_the_queues(B, O):
+    """One row, 2^18 columns: the queues hold fewer words than the bitmap of
+    expandable vertices, which then has memory of its own from the start."""
+    torch = torch_cuda()
+    rng = np.random.default_rng(4)
+    n = 1 << 18
+    indptr = np.full(n + 1, 6000, np.uint32)
+    indptr[0] = 0
+    graphs = [B.Csc(indptr, rng.integers(0, n, 6000), 1, n) for _ in range(2)]
+    batch = B.MultiBatch(graphs)
+    out = torch.empty(2 * n, dtype=torch.int32, device="cuda")
+    for roots in ([0, 0], [0, 77]):
+        refs = [O.oracle_bfs_queue(g.indptr, g.inds, r, 1, n) for g, r in zip(graphs, roots)]
+        for cfg in ((128, 1, 1), (512, 2, 1), (256, 4, 2), (512, 2, 8)):
+            out.fill_(5)
+            ec, _ = batch.run(roots, out.data_ptr(), *cfg)
+            lv = out.cpu().numpy()
+            for i, (ref, edges) in enumerate(refs):
+                assert np.array_equal(lv[i * n:(i + 1) * n], ref) and ec[i] == edges, (cfg, i)
+    batch.free()
